@@ -837,6 +837,8 @@ __global__ void __launch_bounds__((W + NP) * 32) k_f32split(ComputeArgs a)
                         }
                     }
                 }
+                // the row's threads zero their sums for the next item only now
+                __syncwarp();
             }
             PH_MARK(PH_END);
         }
