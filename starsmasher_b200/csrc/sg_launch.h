@@ -178,12 +178,13 @@ cudaError_t launch_wtile_out(const SetDesc *sets, const int *tile_set, int ntile
 // rlist[S.ioff, S.ioff + rcount[s]) in tiles of `itile` rows, every tile
 // split into the same number of j-chunks (enough items to fill `target`
 // persistent blocks, at least 256 sources per chunk), one partial slot per
-// item.  Writes rsets (copies of sets with ni, ntiles, nchunks, slot_off of
-// the refine), the items and their count.  At most max_items items are
-// written; a plan that would need more sets DEVERR_INPUT (never expected:
-// the host sizes max_items for every row flagged).
-// Row-chunk items (sets with at most 32 listed rows: one warp per row and
-// source chunk) a refine plan may hold.
+// item; sets with at most 32 listed rows take row-chunk items instead (one warp
+// per row and source chunk), unless all of them together list more than
+// REFINE_LIGHT_CAP rows.  Writes rsets (copies of sets with ni, ntiles, nchunks,
+// slot_off of the refine), the items and their count.  At most max_items items
+// are written; a plan that would need more sets DEVERR_INPUT (never expected:
+// the host sizes max_items for every row flagged, in tiles).
+// Row-chunk items that a refine plan may hold.
 constexpr int REFINE_LIGHT_CAP = 65536;
 cudaError_t launch_refine_plan(const SetDesc *sets, int nsets, const int *rcount, int itile,
                                int tj, int min_j, int target, int max_items, SetDesc *rsets,

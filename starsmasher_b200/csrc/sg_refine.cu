@@ -89,18 +89,32 @@ __global__ void __launch_bounds__(PLAN_NT) k_refine_plan(const SetDesc *sets, in
     const int t = threadIdx.x;
     const int per = (nsets + blockDim.x - 1) / blockDim.x;
     const int s0 = min(nsets, t * per), s1 = min(nsets, s0 + per);
-    auto light = [&](int r) { return r > 0 && r <= REFINE_LIGHT_ROWS; };
+    int light_most = REFINE_LIGHT_ROWS;
+    auto light = [&](int r) { return r > 0 && r <= light_most; };
     // pass 1: refine tiles, light rows and merge units of this thread's sets
-    long long tiles = 0, lrows = 0, units = 0;
+    long long tiles = 0, lrows = 0, ltiles = 0, units = 0;
     for (int s = s0; s < s1; s++) {
-        const int r = min(rcount[s], sets[s].ni);
-        if (light(r)) lrows += r;
-        else tiles += (r + itile - 1) / itile;
+        const int r = min(rcount[s], sets[s].ni), nt = (r + itile - 1) / itile;
+        if (light(r)) {
+            lrows += r;
+            ltiles += nt;
+        } else {
+            tiles += nt;
+        }
         units += (r + MERGE_ROWS - 1) / MERGE_ROWS;
     }
     long long total_tiles = 0, total_lrows = 0, total_units = 0;
     block_exclusive_scan(tiles, &total_tiles);
     block_exclusive_scan(lrows, &total_lrows);
+    if (total_lrows > REFINE_LIGHT_CAP) {
+        // more light rows (of thousands of sets) than row-chunk items: all sets
+        // take tiles, which fill the GPU then and for which max_items suffices
+        long long more = 0;
+        block_exclusive_scan(ltiles, &more);
+        total_tiles += more;
+        total_lrows = 0;
+        light_most = 0;
+    }
     long long ubase = block_exclusive_scan(units, &total_units);
     const int nch_global = total_tiles > 0 ? (int)max(1ll, (long long)target / total_tiles) : 1;
     const int nchl_global =

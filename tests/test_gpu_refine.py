@@ -55,6 +55,23 @@ def test_refine_of_a_batch_with_both_routes():
     assert np.allclose(a[3], b[3], rtol=1e-6) and np.allclose(a[4], b[4], rtol=1e-6)
 
 
+@pytest.mark.parametrize("nsets", [2048, 2049, 2100])
+def test_more_light_rows_than_row_chunk_items(nsets):
+    """Sets of 32 rows, all listed: 65,536 row-chunk items hold 2,048 of them."""
+    base = inputs.single_polytrope(96, 1.5, seed=5)
+    x, y, z, m, r2 = (np.tile(getattr(base, f)[:32], nsets) for f in ("x", "y", "z", "m", "range2"))
+    x = x * (1.0 + 1e-3 * np.repeat(np.arange(nsets) % 7, 32))  # not one set over and over
+    r2 = 0.01 * r2
+    offs = 32 * np.arange(nsets + 1)
+    with Context(0) as ctx:
+        ctx.set_refine(1e-9)
+        a = ctx.batch_forces(offs, x, y, z, m, r2, 0, "f32split")
+        assert ctx.last_refine_rows() == 32 * nsets
+        b = ctx.batch_forces(offs, x, y, z, m, r2, 0, "fp64")
+    _check(a[:4], b[:4])
+    assert np.allclose(a[4], b[4], rtol=1e-12)
+
+
 @pytest.mark.parametrize("n", [3001, 20011, 60000])
 @pytest.mark.parametrize("refine", [1.0, 0.0])
 def test_point_mass_core(n, refine):
