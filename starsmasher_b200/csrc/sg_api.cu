@@ -983,7 +983,10 @@ static int run_device(sphgrav_ctx *c, const std::vector<int> &offsets, bool full
     TRY(prepare(c, offsets, full_rows, i_lo, ni, precision, variant));
     const Plan &P = c->plan;
     cudaStream_t st = c->stream;
-    if (P.ntot == 0) return SPHGRAV_OK;
+    if (P.ntot == 0) {  // no launch: W of empty sets
+        if (W) CUDA_TRY(cudaMemsetAsync(W, 0, sizeof(double) * P.nsets, st));
+        return SPHGRAV_OK;
+    }
     SortedF64 D = sorted64(c);
     SortedF32 F = sorted32(c);
     const bool refine = precision == SPHGRAV_F32SPLIT && c->refine_T > 0.0;
@@ -1416,7 +1419,6 @@ int sphgrav_forces_device(sphgrav_ctx *c, int n, int i_begin, int ni, const doub
     const bool full = (i_begin == 0 && ni == n);
     InputsDev in = {x, y, z, mass, range2};
     OutputsDev out = {ax, ay, az, pot};
-    if (W && n == 0) CUDA_TRY(cudaMemsetAsync(W, 0, sizeof(double), c->stream));
     return run_device(c, offs, full, i_begin, ni, in, out, W, nkernel, precision);
 }
 

@@ -41,3 +41,14 @@ def test_alternating_calls_repeat_bit_for_bit():
         for k in (0, 3, 1, 4, 2, 5, 0, 5, 3):
             got = ctx.forces(*arrays(calls[k][0]), 0, calls[k][1])
             assert all(np.array_equal(a, b) for a, b in zip(got, want[k])), k
+
+
+@pytest.mark.parametrize("precision", ["fp64", "f32split", "tree"])
+def test_w_of_empty_sets(precision):
+    s = inputs.single_polytrope(300, 1.5, seed=3)
+    none = [np.zeros(0)] * 5
+    with Context(0) as ctx:
+        full = ctx.batch_forces([0, 100, 200, 300], s.x, s.y, s.z, s.m, s.range2, 0, precision)
+        assert (full[4] < 0.0).all()
+        empty = ctx.batch_forces([0, 0, 0, 0], *none, 0, precision)
+        assert not empty[4].any()
