@@ -34,6 +34,10 @@ inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+// Kernels with a set per block row loop over the sets that a grid's second
+// dimension (at most 65,535) cannot number.
+inline unsigned grid_sets(int nsets) { return nsets < 65535 ? nsets : 65535; }
+
 // Input arrays in the caller's (original) order, device pointers.
 struct InputsDev {
     const double *x, *y, *z, *m, *r2;

@@ -40,58 +40,58 @@ __global__ void __launch_bounds__(256) k_bbox(const SetDesc *sets, int nsets, In
 {
     __shared__ unsigned long long s_box[8][6];
     pdl_enter();
-    if (blockIdx.x == 0) {
-        const int s = blockIdx.y;
-        if (s == 0 && threadIdx.x == 0) {
-            *cnt.head = 0;
-            if (cnt.rhead) *cnt.rhead = 0;
-        }
-        if (cnt.rcount && threadIdx.x == 0) cnt.rcount[s] = 0;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+        *cnt.head = 0;
+        if (cnt.rhead) *cnt.rhead = 0;
     }
-    const SetDesc S = sets[blockIdx.y];
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    bool bad = false;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S.n; k += gridDim.x * blockDim.x) {
-        const int p = S.off + k;
-        const double v[3] = {in.x[p], in.y[p], in.z[p]};
-        const double m = in.m[p], r2 = in.r2[p];
-        bad |= !(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]) && isfinite(m) && m > 0.0 &&
-                 isfinite(r2) && r2 != 0.0);
+    for (int s = blockIdx.y; s < nsets; s += gridDim.y) {
+        if (cnt.rcount && blockIdx.x == 0 && threadIdx.x == 0) cnt.rcount[s] = 0;
+        const SetDesc S = sets[s];
+        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        bool bad = false;
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S.n; k += gridDim.x * blockDim.x) {
+            const int p = S.off + k;
+            const double v[3] = {in.x[p], in.y[p], in.z[p]};
+            const double m = in.m[p], r2 = in.r2[p];
+            bad |= !(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]) && isfinite(m) && m > 0.0 &&
+                     isfinite(r2) && r2 != 0.0);
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                lo[d] = fmin(lo[d], v[d]);
+                hi[d] = fmax(hi[d], v[d]);
+            }
+        }
+        if (bad) atomicOr(err, DEVERR_INPUT);
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            lo[d] = fmin(lo[d], v[d]);
-            hi[d] = fmax(hi[d], v[d]);
+            for (int o = 16; o > 0; o >>= 1) {
+                lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+                hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+            }
         }
-    }
-    if (bad) atomicOr(err, DEVERR_INPUT);
+        if (s != (int)blockIdx.y) __syncthreads();  // the previous set's box has been read
+        if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+            for (int d = 0; d < 3; d++) {
+                const bool any = lo[d] <= hi[d];
+                s_box[threadIdx.x >> 5][d] = any ? dkey(lo[d]) : ~0ull;
+                s_box[threadIdx.x >> 5][3 + d] = any ? ~dkey(hi[d]) : ~0ull;
+            }
         }
-    }
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const bool any = lo[d] <= hi[d];
-            s_box[threadIdx.x >> 5][d] = any ? dkey(lo[d]) : ~0ull;
-            s_box[threadIdx.x >> 5][3 + d] = any ? ~dkey(hi[d]) : ~0ull;
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            unsigned long long v = s_box[0][threadIdx.x];
+            for (int w = 1; w < (int)(blockDim.x >> 5); w++) v = min(v, s_box[w][threadIdx.x]);
+            if (v != ~0ull) atomicMin(bbox + 6 * (size_t)s + threadIdx.x, v);
         }
-    }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        unsigned long long v = s_box[0][threadIdx.x];
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) v = min(v, s_box[w][threadIdx.x]);
-        if (v != ~0ull) atomicMin(bbox + 6 * (size_t)blockIdx.y + threadIdx.x, v);
     }
 }
 
 cudaError_t launch_bbox(const SetDesc *sets, int nsets, int max_n, const InputsDev &in,
                         unsigned long long *bbox, const Counters &cnt, int *err, cudaStream_t st)
 {
-    return launch(k_bbox, dim3(grid_for(max_n, 256, 296), nsets), 256, 0, st, sets, nsets, in, bbox,
-                  cnt, err);
+    return launch(k_bbox, dim3(grid_for(max_n, 256, 296), grid_sets(nsets)), 256, 0, st, sets, nsets, in,
+                  bbox, cnt, err);
 }
 
 // ----------------------------------------------------------- Hilbert keys
@@ -172,17 +172,19 @@ __device__ __forceinline__ unsigned long long sfc_key(const InputsDev &in, int p
     return ((unsigned long long)s << (3 * bits)) | hilbert3(q[0], q[1], q[2], bits);
 }
 
-__global__ void k_sfc_keys(const SetDesc *sets, InputsDev in, const unsigned long long *bbox,
-                           int bits, unsigned long long *keys, int *vals)
+__global__ void k_sfc_keys(const SetDesc *sets, int nsets, InputsDev in,
+                           const unsigned long long *bbox, int bits, unsigned long long *keys,
+                           int *vals)
 {
     pdl_enter();
-    const int s = blockIdx.y;
-    const SetDesc S = sets[s];
-    const KeyScale K = key_scale(bbox, s, bits);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S.n; k += gridDim.x * blockDim.x) {
-        const int p = S.off + k;
-        keys[p] = sfc_key(in, p, s, K, bits);
-        vals[p] = p;
+    for (int s = blockIdx.y; s < nsets; s += gridDim.y) {
+        const SetDesc S = sets[s];
+        const KeyScale K = key_scale(bbox, s, bits);
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S.n; k += gridDim.x * blockDim.x) {
+            const int p = S.off + k;
+            keys[p] = sfc_key(in, p, s, K, bits);
+            vals[p] = p;
+        }
     }
 }
 
@@ -315,8 +317,9 @@ cudaError_t launch_sorted(const SetDesc *sets, int nsets, int max_n, int ntot, c
         return launch(k_tile_rank, (ntot + 255) / 256, 256, 0, st, ntot, keys_in, vals_in, keys_out,
                       vals_out);
     }
-    const dim3 grid(grid_for(max_n, 256, 1024), nsets);
-    const cudaError_t e = launch(k_sfc_keys, grid, 256, 0, st, sets, in, bbox, bits, keys_in, vals_in);
+    const dim3 grid(grid_for(max_n, 256, 1024), grid_sets(nsets));
+    const cudaError_t e = launch(k_sfc_keys, grid, 256, 0, st, sets, nsets, in, bbox, bits, keys_in,
+                                 vals_in);
     if (e != cudaSuccess) return e;
     // CUB's onesweep radix sort: a handful of kernels per call.
     g_launches += 1 + (end_bit + 7) / 8;
@@ -325,57 +328,60 @@ cudaError_t launch_sorted(const SetDesc *sets, int nsets, int max_n, int ntot, c
 }
 
 // ------------------------------------------------------------------ gather
-__global__ void k_gather(const SetDesc *sets, InputsDev in, const int *sorted_vals,
+__global__ void k_gather(const SetDesc *sets, int nsets, InputsDev in, const int *sorted_vals,
                          SortedF64 D, SortedF32 F, int *ilist, unsigned long long *bbox)
 {
     pdl_enter();
-    const SetDesc S = sets[blockIdx.y];
-    if (blockIdx.x == 0 && threadIdx.x < 6) bbox[6 * (size_t)blockIdx.y + threadIdx.x] = ~0ull;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S.npad; k += gridDim.x * blockDim.x) {
-        const int slot = S.poff + k;
-        if (k < S.n) {
-            const int p = sorted_vals[S.off + k];
-            if (ilist) ilist[S.ioff + k] = slot;
-            const double x = in.x[p], y = in.y[p], z = in.z[p], m = in.m[p], r2 = in.r2[p];
-            D.x[slot] = x;
-            D.y[slot] = y;
-            D.z[slot] = z;
-            D.m[slot] = m;
-            const double h2 = fabs(r2), h = __dsqrt_rn(h2), mh = __ddiv_rn(m, h);
-            D.h2[slot] = h2;
-            D.h[slot] = h;
-            D.mh[slot] = mh;
-            D.mh3[slot] = __ddiv_rn(mh, h2);
-            D.orig[slot] = p;
-            D.flag[slot] = r2 > 0.0 ? 1 : 0;
-            // split of the FP64 positions into float hi + lo pairs
-            const float xh = __double2float_rn(x), yh = __double2float_rn(y),
-                        zh = __double2float_rn(z);
-            F.xh[slot] = xh;
-            F.xl[slot] = __double2float_rn(x - (double)xh);
-            F.yh[slot] = yh;
-            F.yl[slot] = __double2float_rn(y - (double)yh);
-            F.zh[slot] = zh;
-            F.zl[slot] = __double2float_rn(z - (double)zh);
-            F.m[slot] = __double2float_rn(m);
-            F.h2[slot] = __double2float_rn(fabs(r2));
-        } else {
-            D.x[slot] = FAR_POS;
-            D.y[slot] = FAR_POS;
-            D.z[slot] = FAR_POS;
-            D.m[slot] = 0.0;
-            D.h2[slot] = 0.0;
-            D.h[slot] = D.mh[slot] = D.mh3[slot] = 0.0;
-            D.orig[slot] = -1;
-            D.flag[slot] = 0;
-            F.xh[slot] = (float)FAR_POS;
-            F.xl[slot] = 0.f;
-            F.yh[slot] = (float)FAR_POS;
-            F.yl[slot] = 0.f;
-            F.zh[slot] = (float)FAR_POS;
-            F.zl[slot] = 0.f;
-            F.m[slot] = 0.f;
-            F.h2[slot] = 0.f;
+    for (int s = blockIdx.y; s < nsets; s += gridDim.y) {
+        const SetDesc S = sets[s];
+        if (blockIdx.x == 0 && threadIdx.x < 6) bbox[6 * (size_t)s + threadIdx.x] = ~0ull;
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < S.npad;
+             k += gridDim.x * blockDim.x) {
+            const int slot = S.poff + k;
+            if (k < S.n) {
+                const int p = sorted_vals[S.off + k];
+                if (ilist) ilist[S.ioff + k] = slot;
+                const double x = in.x[p], y = in.y[p], z = in.z[p], m = in.m[p], r2 = in.r2[p];
+                D.x[slot] = x;
+                D.y[slot] = y;
+                D.z[slot] = z;
+                D.m[slot] = m;
+                const double h2 = fabs(r2), h = __dsqrt_rn(h2), mh = __ddiv_rn(m, h);
+                D.h2[slot] = h2;
+                D.h[slot] = h;
+                D.mh[slot] = mh;
+                D.mh3[slot] = __ddiv_rn(mh, h2);
+                D.orig[slot] = p;
+                D.flag[slot] = r2 > 0.0 ? 1 : 0;
+                // split of the FP64 positions into float hi + lo pairs
+                const float xh = __double2float_rn(x), yh = __double2float_rn(y),
+                            zh = __double2float_rn(z);
+                F.xh[slot] = xh;
+                F.xl[slot] = __double2float_rn(x - (double)xh);
+                F.yh[slot] = yh;
+                F.yl[slot] = __double2float_rn(y - (double)yh);
+                F.zh[slot] = zh;
+                F.zl[slot] = __double2float_rn(z - (double)zh);
+                F.m[slot] = __double2float_rn(m);
+                F.h2[slot] = __double2float_rn(fabs(r2));
+            } else {
+                D.x[slot] = FAR_POS;
+                D.y[slot] = FAR_POS;
+                D.z[slot] = FAR_POS;
+                D.m[slot] = 0.0;
+                D.h2[slot] = 0.0;
+                D.h[slot] = D.mh[slot] = D.mh3[slot] = 0.0;
+                D.orig[slot] = -1;
+                D.flag[slot] = 0;
+                F.xh[slot] = (float)FAR_POS;
+                F.xl[slot] = 0.f;
+                F.yh[slot] = (float)FAR_POS;
+                F.yl[slot] = 0.f;
+                F.zh[slot] = (float)FAR_POS;
+                F.zl[slot] = 0.f;
+                F.m[slot] = 0.f;
+                F.h2[slot] = 0.f;
+            }
         }
     }
 }
@@ -384,8 +390,8 @@ cudaError_t launch_gather(const SetDesc *sets, int nsets, int max_npad, const In
                           const int *sorted_vals, SortedF64 D, SortedF32 F, int *ilist,
                           unsigned long long *bbox, cudaStream_t st)
 {
-    dim3 grid(grid_for(max_npad, 256, 1024), nsets);
-    return launch(k_gather, grid, 256, 0, st, sets, in, sorted_vals, D, F, ilist, bbox);
+    const dim3 grid(grid_for(max_npad, 256, 1024), grid_sets(nsets));
+    return launch(k_gather, grid, 256, 0, st, sets, nsets, in, sorted_vals, D, F, ilist, bbox);
 }
 
 // ---------------------------------------------------------------- row list

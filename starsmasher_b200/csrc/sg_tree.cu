@@ -72,41 +72,43 @@ __device__ __forceinline__ int back(int hi, int lo, int o, int lane)
     return lane >= o ? h : l;
 }
 
-__global__ void k_tree_bits(const SetDesc *sets, int levels, const unsigned long long *keys,
-                            int ngrp, unsigned *bits, int *cnt)
+__global__ void k_tree_bits(const SetDesc *sets, int nroots, int levels,
+                            const unsigned long long *keys, int ngrp, unsigned *bits, int *cnt)
 {
     static_assert(TREE_LEAF == 16, "the window maximum below is 17 positions wide");
-    const SetDesc S = sets[blockIdx.y];
     const int lane = threadIdx.x & 31;
     const int k0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) cnt[levels * ngrp] = 0;
-    if (k0 >= S.npad) return;
-    const unsigned long long *key = keys + S.off;
-    // shared digits of positions w and w + 16, for the warp's positions and the 16 before
-    auto window = [&](int w) {
-        return w >= 0 && w + TREE_LEAF < S.n ? common_digits(key[w], key[w + TREE_LEAF], levels) : -1;
-    };
-    int hi = window(k0 + lane), lo = window(k0 - 32 + lane);
+    for (int set = blockIdx.y; set < nroots; set += gridDim.y) {
+        const SetDesc S = sets[set];
+        if (k0 >= S.npad) continue;
+        const unsigned long long *key = keys + S.off;
+        // shared digits of positions w and w + 16, for the warp's positions and the 16 before
+        auto window = [&](int w) {
+            return w >= 0 && w + TREE_LEAF < S.n ? common_digits(key[w], key[w + TREE_LEAF], levels) : -1;
+        };
+        int hi = window(k0 + lane), lo = window(k0 - 32 + lane);
 #pragma unroll
-    for (int o = 1; o <= 8; o <<= 1) {  // maximum over 2, 4, 8, 16 positions back
-        const int h = back(hi, lo, o, lane);
-        const int l = __shfl_up_sync(0xffffffffu, lo, o);
-        hi = max(hi, h);
-        if (lane >= o) lo = max(lo, l);
-    }
-    const int deepest = max(hi, back(hi, lo, 1, lane)) + 1;
-    const int k = k0 + lane;
-    int first = levels + 1;
-    if (k < S.n) first = k == 0 ? 1 : common_digits(key[k - 1], key[k], levels) + 1;
-    unsigned mine = 0u;
-    for (int L = 1; L <= levels; L++) {
-        const unsigned m = __ballot_sync(0xffffffffu, first <= L && L <= deepest);
-        if (lane == L - 1) mine = m;
-    }
-    if (lane < levels) {
-        const size_t g = (size_t)lane * ngrp + S.poff / 32 + k0 / 32;
-        bits[g] = mine;
-        cnt[g] = __popc(mine);
+        for (int o = 1; o <= 8; o <<= 1) {  // maximum over 2, 4, 8, 16 positions back
+            const int h = back(hi, lo, o, lane);
+            const int l = __shfl_up_sync(0xffffffffu, lo, o);
+            hi = max(hi, h);
+            if (lane >= o) lo = max(lo, l);
+        }
+        const int deepest = max(hi, back(hi, lo, 1, lane)) + 1;
+        const int k = k0 + lane;
+        int first = levels + 1;
+        if (k < S.n) first = k == 0 ? 1 : common_digits(key[k - 1], key[k], levels) + 1;
+        unsigned mine = 0u;
+        for (int L = 1; L <= levels; L++) {
+            const unsigned m = __ballot_sync(0xffffffffu, first <= L && L <= deepest);
+            if (lane == L - 1) mine = m;
+        }
+        if (lane < levels) {
+            const size_t g = (size_t)lane * ngrp + S.poff / 32 + k0 / 32;
+            bits[g] = mine;
+            cnt[g] = __popc(mine);
+        }
     }
 }
 
@@ -130,70 +132,71 @@ __global__ void k_tree_emit(const SetDesc *sets, int nroots, int levels,
         if (L == 0) lv[TREE_LV_OVERFLOW] = full ? (int)min(total, 0x7fffffffll) : 0;
     }
     if (full) return;
-    const int set = blockIdx.y;
-    const SetDesc S = sets[set];
     const int k0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
-    if (k0 > 0 && k0 >= S.n) return;
-    const unsigned long long *key = keys + S.off;
-    const int k = k0 + lane;
-    const int g = S.poff / 32 + k0 / 32;
-    const unsigned below = (1u << lane) - 1u;
-    // nodes of level L that start before position p
-    auto rank = [&](int L, int p) {
-        const int q = S.poff + p, h = (L - 1) * ngrp + (q >> 5);
-        int r = off[h];
-        if (q & 31) r += __popc(bits[h] & ((1u << (q & 31)) - 1u));
-        return nroots + r;
-    };
-    auto write = [&](int i, int start, int end, int L, int child) {
-        TreeNode T;
-        T.start = S.poff + start;
-        T.end = S.poff + end;
-        T.child = 0;
-        T.nchild = 0;
-        if (child >= 0) {
-            T.child = child;
-            T.nchild = rank(L + 1, end) - child;
-            for (int c = 0; c < T.nchild; c++) parent[child + c] = i;
-        }
-        nodes[i] = T;
-        done[i] = 0;
-    };
-    int child = -1;  // this position's node one level down
-    int end = k + 1;
-    for (int L = levels; L >= 1; L--) {
-        const int h = (L - 1) * ngrp + g;
-        const unsigned m = k0 < S.npad ? bits[h] : 0u;
-        if (m == 0u) continue;
-        if (!((m >> lane) & 1u)) {
-            child = -1;
-            continue;
-        }
-        // end of the cell: first position whose first L digits differ, by
-        // galloping from the end of the cell one level down
-        const int sh = 3 * (levels - L);
-        const unsigned long long v = key[k] >> sh;
-        int step = 1;
-        while (end < S.n && (key[end] >> sh) == v) {
-            end += step;
-            step <<= 1;
-        }
-        if (step > 1) {  // the last probe that matched: end - step / 2
-            int lo = end - (step >> 1) + 1, hi = min(end, S.n);
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if ((key[mid] >> sh) == v) lo = mid + 1;
-                else hi = mid;
+    for (int set = blockIdx.y; set < nroots; set += gridDim.y) {
+        const SetDesc S = sets[set];
+        if (k0 > 0 && k0 >= S.n) continue;
+        const unsigned long long *key = keys + S.off;
+        const int k = k0 + lane;
+        const int g = S.poff / 32 + k0 / 32;
+        const unsigned below = (1u << lane) - 1u;
+        // nodes of level L that start before position p
+        auto rank = [&](int L, int p) {
+            const int q = S.poff + p, h = (L - 1) * ngrp + (q >> 5);
+            int r = off[h];
+            if (q & 31) r += __popc(bits[h] & ((1u << (q & 31)) - 1u));
+            return nroots + r;
+        };
+        auto write = [&](int i, int start, int end, int L, int child) {
+            TreeNode T;
+            T.start = S.poff + start;
+            T.end = S.poff + end;
+            T.child = 0;
+            T.nchild = 0;
+            if (child >= 0) {
+                T.child = child;
+                T.nchild = rank(L + 1, end) - child;
+                for (int c = 0; c < T.nchild; c++) parent[child + c] = i;
             }
-            end = lo;
+            nodes[i] = T;
+            done[i] = 0;
+        };
+        int child = -1;  // this position's node one level down
+        int end = k + 1;
+        for (int L = levels; L >= 1; L--) {
+            const int h = (L - 1) * ngrp + g;
+            const unsigned m = k0 < S.npad ? bits[h] : 0u;
+            if (m == 0u) continue;
+            if (!((m >> lane) & 1u)) {
+                child = -1;
+                continue;
+            }
+            // end of the cell: first position whose first L digits differ, by
+            // galloping from the end of the cell one level down
+            const int sh = 3 * (levels - L);
+            const unsigned long long v = key[k] >> sh;
+            int step = 1;
+            while (end < S.n && (key[end] >> sh) == v) {
+                end += step;
+                step <<= 1;
+            }
+            if (step > 1) {  // the last probe that matched: end - step / 2
+                int lo = end - (step >> 1) + 1, hi = min(end, S.n);
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if ((key[mid] >> sh) == v) lo = mid + 1;
+                    else hi = mid;
+                }
+                end = lo;
+            }
+            const int i = nroots + off[h] + __popc(m & below);
+            write(i, k, end, L, end - k > TREE_LEAF && L < levels ? child : -1);
+            child = i;
         }
-        const int i = nroots + off[h] + __popc(m & below);
-        write(i, k, end, L, end - k > TREE_LEAF && L < levels ? child : -1);
-        child = i;
-    }
-    if (k == 0) {
-        parent[set] = -1;
-        write(set, 0, S.n, 0, S.n > TREE_LEAF ? child : -1);
+        if (k == 0) {
+            parent[set] = -1;
+            write(set, 0, S.n, 0, S.n > TREE_LEAF ? child : -1);
+        }
     }
 }
 
@@ -931,41 +934,44 @@ cudaError_t tree_heavy(int nheavy_host, const int *nheavy, int cap, const int *h
 // the set's slots (a contiguous run, in a fixed order) for W.
 constexpr int SCATTER_NT = 256;
 __global__ void __launch_bounds__(SCATTER_NT)
-k_tree_scatter(const SetDesc *sets, int nslots, bool split, int i_lo, int ni, const double *res,
-               SortedF64 D, OutputsDev out, double *wpart)
+k_tree_scatter(const SetDesc *sets, int nsets, int nslots, bool split, int i_lo, int ni,
+               const double *res, SortedF64 D, OutputsDev out, double *wpart)
 {
     __shared__ double s_w[SCATTER_NT];
-    const SetDesc S = sets[blockIdx.y];
-    const int nparts = split ? tree_walk_parts(S.n) : 1;
-    const int per = ((S.n + gridDim.x - 1) / gridDim.x + SCATTER_NT - 1) / SCATTER_NT * SCATTER_NT;
-    const int k0 = min(S.n, (int)min((long long)S.n, (long long)blockIdx.x * per));
-    const int k1 = min(S.n, k0 + per);
-    double w = 0.0;
-    for (int k = k0 + threadIdx.x; k < k1; k += SCATTER_NT) {
-        const int s = S.poff + k;
-        double v[4];
+    for (int set = blockIdx.y; set < nsets; set += gridDim.y) {
+        const SetDesc S = sets[set];
+        const int nparts = split ? tree_walk_parts(S.n) : 1;
+        const int per = ((S.n + gridDim.x - 1) / gridDim.x + SCATTER_NT - 1) / SCATTER_NT * SCATTER_NT;
+        const int k0 = min(S.n, (int)min((long long)S.n, (long long)blockIdx.x * per));
+        const int k1 = min(S.n, k0 + per);
+        double w = 0.0;
+        for (int k = k0 + threadIdx.x; k < k1; k += SCATTER_NT) {
+            const int s = S.poff + k;
+            double v[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) v[q] = res[(size_t)q * nslots + s];
-        for (int p = 1; p < nparts; p++) {
+            for (int q = 0; q < 4; q++) v[q] = res[(size_t)q * nslots + s];
+            for (int p = 1; p < nparts; p++) {
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] += res[((size_t)p * 4 + q) * nslots + s];
+                for (int q = 0; q < 4; q++) v[q] += res[((size_t)p * 4 + q) * nslots + s];
+            }
+            w += D.m[s] * v[3];
+            const int o = D.orig[s];
+            if (o < i_lo || o >= i_lo + ni) continue;
+            out.ax[o] = v[0];
+            out.ay[o] = v[1];
+            out.az[o] = v[2];
+            out.pot[o] = v[3];
         }
-        w += D.m[s] * v[3];
-        const int o = D.orig[s];
-        if (o < i_lo || o >= i_lo + ni) continue;
-        out.ax[o] = v[0];
-        out.ay[o] = v[1];
-        out.az[o] = v[2];
-        out.pot[o] = v[3];
-    }
-    if (!wpart) return;
-    s_w[threadIdx.x] = w;
-    __syncthreads();
-    for (int o = SCATTER_NT / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) s_w[threadIdx.x] += s_w[threadIdx.x + o];
+        if (!wpart) continue;
+        __syncthreads();  // the previous set's sum has been read
+        s_w[threadIdx.x] = w;
         __syncthreads();
+        for (int o = SCATTER_NT / 2; o > 0; o >>= 1) {
+            if ((int)threadIdx.x < o) s_w[threadIdx.x] += s_w[threadIdx.x + o];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) wpart[(size_t)set * gridDim.x + blockIdx.x] = s_w[0];
     }
-    if (threadIdx.x == 0) wpart[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s_w[0];
 }
 
 // W = 1/2 sum m phi of every set from its blocks' sums: one block per set, fixed order.
@@ -1006,9 +1012,9 @@ size_t tree_scan_temp_bytes(int n)
 cudaError_t tree_build(const TreeBuildArgs &t, cudaStream_t st)
 {
     const int ngrp = t.nslots / 32;
-    const dim3 grid((t.max_npad / 32 + 7) / 8, t.nroots);
+    const dim3 grid((t.max_npad / 32 + 7) / 8, grid_sets(t.nroots));
     if (ngrp > 0) {
-        k_tree_bits<<<grid, 256, 0, st>>>(t.sets, t.levels, t.keys, ngrp, t.bits, t.cnt);
+        k_tree_bits<<<grid, 256, 0, st>>>(t.sets, t.nroots, t.levels, t.keys, ngrp, t.bits, t.cnt);
         ++g_launches;
         size_t tb = t.scan_temp_bytes;
         const cudaError_t e = cub::DeviceScan::ExclusiveSum(t.scan_temp, tb, t.cnt, t.off,
@@ -1116,8 +1122,8 @@ cudaError_t tree_scatter(const SetDesc *sets, int nsets, int max_n, int nslots, 
                          double *wpart, double *W, cudaStream_t st)
 {
     const int nb = tree_scatter_blocks(max_n);
-    k_tree_scatter<<<dim3(nb, nsets), SCATTER_NT, 0, st>>>(sets, nslots, nparts > 1, i_lo, ni, res, D,
-                                                           out, W ? wpart : nullptr);
+    k_tree_scatter<<<dim3(nb, grid_sets(nsets)), SCATTER_NT, 0, st>>>(
+        sets, nsets, nslots, nparts > 1, i_lo, ni, res, D, out, W ? wpart : nullptr);
     ++g_launches;
     if (W) {
         k_tree_wsum<<<nsets, SCATTER_NT, 0, st>>>(nb, wpart, W);

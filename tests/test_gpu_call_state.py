@@ -52,3 +52,22 @@ def test_w_of_empty_sets(precision):
         assert (full[4] < 0.0).all()
         empty = ctx.batch_forces([0, 0, 0, 0], *none, 0, precision)
         assert not empty[4].any()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "f32split", "tree"])
+def test_more_sets_than_a_grid_dimension(precision):
+    """Batches may hold 2^20 sets; a grid's second dimension ends at 65,535."""
+    pairs = 66001
+    rng = np.random.default_rng(1)
+    d, m = rng.uniform(0.5, 2.0, pairs), rng.uniform(0.1, 1.0, 2 * pairs)
+    x = np.zeros(2 * pairs)
+    x[1::2] = d  # two point masses in each set, farther apart than their H
+    zero, r2 = np.zeros(2 * pairs), np.full(2 * pairs, -0.01)
+    offs = np.concatenate([[0, 0], 2 * np.arange(1, pairs + 1)])  # the first set is empty
+    with Context(0) as ctx:
+        ax, ay, az, pot, w = ctx.batch_forces(offs, x, zero, zero, m, r2, 0, precision)
+    want = np.empty_like(x)
+    want[0::2], want[1::2] = m[1::2] / d ** 2, -m[0::2] / d ** 2
+    assert np.allclose(ax, want, rtol=1e-6) and not ay.any() and not az.any()
+    assert np.allclose(pot, -np.abs(want) * np.repeat(d, 2), rtol=1e-6)
+    assert w[0] == 0.0 and np.allclose(w[1:], -m[0::2] * m[1::2] / d, rtol=1e-6)
