@@ -373,21 +373,23 @@ static int choose_variant(sphgrav_ctx *c, int precision, const std::vector<int> 
     //                                 whose 768-row tiles leave more rows beyond
     //                                 8 H of their centre for the FP64
     //                                 refine: 2,357 rows, whole call 37.5 ms)
-    //   from 2^15, and batches from 2^14: W12K1Q2, 7 stages (whole calls; 33K
-    //                                 0.86 vs 0.86 for W15K1Q2, one producer; 50K
-    //                                 collision 1.56 vs 1.70, red giant 1.65 vs
-    //                                 1.77; 90K 4.32 vs 5.02; 16 of 16K-50K 8.21
-    //                                 vs 8.28 for W12K1Q1, whose 384-row tiles
-    //                                 round 6% more, and 9.23 for W12K1Q4)
+    //   single sets from 2^15: W12K1Q2, 7 stages (whole calls; 33K 0.86 vs 0.86 for
+    //                                 W15K1Q2, one producer; 50K collision 1.56 vs
+    //                                 1.70, red giant 1.65 vs 1.77; 90K 4.32 vs
+    //                                 5.02).  Batches keep W12K1Q4 there: over ten
+    //                                 batches with a mean of 2^14 the 192-row tiles
+    //                                 round 3% more on average (2-norms against
+    //                                 FP64; 40 of 12K-24K 3.73e-8 vs 3.56e-8),
+    //                                 for 8.2 ms a call instead of 9.1
     //   from 2^13: W12K1Q4, 7 stages (8K: 0.135 vs 0.142; 16K: 0.307 vs 0.302
     //                                 for W15K1Q2, whose 240-row tiles leave 69
     //                                 rows for the FP64 refine against 22: whole
-    //                                 call 0.51 vs 0.63 ms), and batches of
-    //                                 smaller sets with a row tile for every SM
-    //                                 (64 of 1K-4K: 813 us vs 985 for W8K1Q4)
+    //                                 call 0.51 vs 0.63 ms)
     //   below    W8K1Q4              (whole calls; 2,000: 88 us vs 94 for
     //                                 W12K1Q4; 5,003: 181 vs 161, but red giant
-    //                                 187 vs 226: more rows refined)
+    //                                 187 vs 226: more rows refined.  Batches: 64
+    //                                 of 1K-4K 0.93 ms vs 0.79 for W12K1Q4, whose
+    //                                 96-row tiles round 2% more on average)
     // Twelve consumer warps put the same number of consumers on every SMSP;
     // all without the Newton step on rsqrt.approx: in FP32 the step's own
     // roundings cost more than it corrects (RMS error 3.2e-8 vs 3.7e-8 at
@@ -403,9 +405,8 @@ static int choose_variant(sphgrav_ctx *c, int precision, const std::vector<int> 
     }
     if (b >= 20 || (batch && b >= 18)) return 0;
     if (b >= 17 || (batch && b >= 15)) return 2;
-    if (b >= 15 || (batch && b >= 14)) return 11;
-    if (b >= 13) return 5;
-    return batch && offsets.back() - offsets.front() >= 148 * 96 ? 5 : 4;
+    if (b >= 15) return 11;
+    return b >= 13 ? 5 : 4;
 }
 
 // ------------------------------------------------------------------ plan
