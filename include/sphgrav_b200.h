@@ -238,7 +238,10 @@ int sphgrav_set_fp64_band(sphgrav_ctx *ctx, double factor);
  * in FP64 on the device in the same call (no host round trip; capturable),
  * so their relative error is that of the FP64 kernel.  Rows lying more than
  * 8 H from the centre of their row tile (where the FP32 rounding of their
- * tile-relative position shifts them measurably) are recomputed too.
+ * tile-relative position shifts them measurably) are recomputed too, and
+ * rows that alone have most of several 256-source tiles within max(H), such
+ * as a point-mass core, whose near pairs the split-FP32 kernel leaves to the
+ * refine.
  * Default 1.0 (0.1-0.4% of the rows of the benchmark workloads); 0 turns the
  * refine off.  No reference counterpart. */
 int sphgrav_set_refine(sphgrav_ctx *ctx, double threshold);

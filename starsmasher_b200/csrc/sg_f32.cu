@@ -297,9 +297,9 @@ constexpr float SHIFT_H = 8.f;
 // core: H = 0.1 holds 70% of the red giant) has 256 near pairs in each of many
 // tiles, eight rounds of near_eval for which its CTA's other warps wait, and
 // usually is recomputed by the refine anyway.  After HEAVY_TILES such tiles of
-// an item, where the refine is on, the row is handed to it (infinite error
-// scale), its sources spread over many warps, and its near pairs are left out
-// from then on.
+// an item, where the refine is on, the row is handed to it (the sign of its
+// G^2 partial), its sources spread over many warps, and its near pairs are left
+// out from then on.
 constexpr int HEAVY_TILES = 4;
 
 // Far tiles whose sources all have one mass (equal-mass models, the usual
@@ -812,12 +812,17 @@ __global__ void __launch_bounds__((W + NP) * 32) k_f32split(ComputeArgs a)
                     for (int k = 0; k < K; k++) {
                         float ga, gb;
                         upk(g2[k], ga, gb);
-                        float gs = heavy < HEAVY_TILES ? ga + gb : INFINITY;
+                        float gs = ga + gb;
+                        bool left_out = heavy >= HEAVY_TILES;  // near pairs, of any of the row's threads
 #pragma unroll
-                        for (int o = 1; o < Q; o <<= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
+                        for (int o = 1; o < Q; o <<= 1) {
+                            gs += __shfl_xor_sync(0xffffffffu, gs, o);
+                            left_out |= __shfl_xor_sync(0xffffffffu, (int)left_out, o) != 0;
+                        }
+                        gs = shifted[k] ? INFINITY : gs * (SA * SA);
                         if (phase == 0 && act[k])
                             a.gpart[slot * ITILE + warp * RPW * K + k * RPW + grp] =
-                                shifted[k] ? INFINITY : gs * (SA * SA);
+                                left_out ? -gs : gs;
                     }
                 }
                 if (phase == 0) {

@@ -95,7 +95,8 @@ struct ComputeArgs {
     double *partials;    // [slot][4][itile], slot = WorkItem::slot
     // split-FP32: [slot][itile] sum over the item's j-tiles of |FP32 tile sum|^2
     // (acceleration components, both packed lanes): the scale of the FP32
-    // rounding error of the row, merged into the refine test (nullable)
+    // rounding error of the row, merged into the refine test (nullable).
+    // Negative: the row's near pairs are not in the item's sums (refine on)
     float *gpart;
     // when non-null the item count is read here instead of `nitems` (work
     // lists planned on the device, e.g. the FP64 refine of flagged rows)
@@ -103,7 +104,7 @@ struct ComputeArgs {
     int *err;
     int nkernel;
     int itile;
-    bool refine;         // split-FP32: rows with an infinite error scale are recomputed in FP64
+    bool refine;         // split-FP32: listed rows are recomputed in FP64 (near pairs may be left to it)
     float band2;         // split-FP32: pairs with r^2 < band2 * max(H^2) use FP64 (>= 1)
     // split-FP32 built with -DSG_PHASES: [PHASE_COUNTERS] clock64 cycles per
     // phase summed over warps (see the Phase enum); nullptr = not counted
@@ -150,7 +151,8 @@ cudaError_t launch_compute(int precision, int v, int grid, const ComputeArgs &a,
 
 // --- merge and diagnostics (sg_prep.cu)
 // Refine test of the merge (split-FP32 calls): rows whose error scale G^2
-// exceeds thresh2 * |a|^2 are listed for the FP64 refine.
+// exceeds thresh2 * |a|^2, or whose near pairs were left out, are listed for the
+// FP64 refine.
 struct MergeRefine {
     const float *gpart = nullptr;  // [slot][itile] G^2 partials; null: no test
     double thresh2 = 0.0;          // T^2

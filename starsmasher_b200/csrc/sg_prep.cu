@@ -609,7 +609,8 @@ __device__ void finish_w(const SetDesc *sets, const WSum &ws)
 // does not depend on which block computed which chunk), scatter to the
 // caller's order, and the per-tile sum of m_i * phi_i in a fixed order.
 // Split-FP32 calls also merge the rows' error scales G^2 (sum over j-tiles of
-// |FP32 tile sum|^2) and append every row with G^2 > thresh2 |a|^2 to its
+// |FP32 tile sum|^2; its sign: the row's near pairs are not in the sums) and
+// append every row with G^2 > thresh2 |a|^2, or without its near pairs, to its
 // set's refine list, rlist[S.ioff + k], k counted in rcount[set].
 constexpr int MERGE_NT = 256;
 constexpr int MERGE_GROUPS = 8;
@@ -638,25 +639,32 @@ __global__ void __launch_bounds__(MERGE_NT) k_merge(const SetDesc *sets, const i
         const int li = l0 + rl;
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
         float g2 = 0.f;
+        bool partial = false;
         for (int g = cg; g < MERGE_GROUPS && li < nrow; g += NCG) {
             double v[4] = {0.0, 0.0, 0.0, 0.0};
             float h = 0.f;
+            bool part = false;  // a chunk without its near pairs
 #pragma unroll 4
             for (int c = g; c < ts.y; c += MERGE_GROUPS) {
                 const size_t slot = (size_t)(ts.x + c);
                 const double *p = partials + slot * 4 * itile;
 #pragma unroll
                 for (int q = 0; q < 4; q++) v[q] += p[q * itile + li];
-                if (R.gpart) h += R.gpart[slot * itile + li];
+                if (R.gpart) {
+                    const float gp = R.gpart[slot * itile + li];
+                    part |= signbit(gp);
+                    h += fabsf(gp);
+                }
             }
             if (NCG > 1) {
 #pragma unroll
                 for (int q = 0; q < 4; q++) s_acc[q][g][rl] = v[q];
-                s_g2[g][rl] = h;
+                s_g2[g][rl] = part ? -h : h;
             } else {
 #pragma unroll
                 for (int q = 0; q < 4; q++) acc[q] += v[q];
                 g2 += h;
+                partial |= part;
             }
         }
         if (NCG > 1) {  // one run: RW >= itile
@@ -665,7 +673,8 @@ __global__ void __launch_bounds__(MERGE_NT) k_merge(const SetDesc *sets, const i
                 for (int g = 0; g < MERGE_GROUPS; g++) {
 #pragma unroll
                     for (int q = 0; q < 4; q++) acc[q] += s_acc[q][g][rl];
-                    g2 += s_g2[g][rl];
+                    g2 += fabsf(s_g2[g][rl]);
+                    partial |= signbit(s_g2[g][rl]);
                 }
             }
         }
@@ -679,7 +688,7 @@ __global__ void __launch_bounds__(MERGE_NT) k_merge(const SetDesc *sets, const i
         w += D.m[slot] * acc[3];
         if (R.gpart) {
             const double a2 = acc[0] * acc[0] + acc[1] * acc[1] + acc[2] * acc[2];
-            if (R.rlist && (double)g2 > R.thresh2 * a2) {
+            if (R.rlist && (partial || (double)g2 > R.thresh2 * a2)) {
                 const int k = atomicAdd(&R.rcount[set], 1);
                 R.rlist[S.ioff + k] = slot;
             }

@@ -9,8 +9,9 @@
 // several 1e-6 even though its absolute error is ordinary.  The kernel also
 // marks (G = infinity) the rows lying more than 8 H from their i-tile centre,
 // whose FP32 tile-relative coordinate is rounded by enough to shift the row
-// measurably.  k_merge lists the rows with G > T |a| per set; this file
-// plans, on the device, an FP64 pass
+// measurably, and leaves out the near pairs of rows that alone have most of
+// several tiles within max(H).  k_merge lists the rows with G > T |a|, and
+// those without their near pairs, per set; this file plans, on the device, an FP64 pass
 // over exactly those rows (k_fp64 over a device-written work list, so the
 // call needs no host round trip and stays graph-capturable) and scatters its
 // results over the FP32 ones.

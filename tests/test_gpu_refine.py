@@ -92,3 +92,24 @@ def test_point_mass_core(n, refine):
     core = np.sqrt(sum((g[0] - r[0]) ** 2 for g, r in zip(got[:3], ref[:3])))
     assert core <= (1e-9 if refine else 1e-6) * np.median(amag)
     assert abs(got[3][0] - ref[3][0]) <= 1e-6 * abs(ref[3][0])
+
+
+@pytest.mark.parametrize("n", [20011, 60000])
+def test_error_scale_of_a_core(n):
+    """The error scale is that of the FP32 tile sums, whether the row's near pairs
+    are in the sums or left to the refine, which then takes the row at any threshold."""
+    s = inputs.red_giant(n, seed=n)
+    a = (s.x, s.y, s.z, s.m, s.range2)
+    G = {}
+    with Context(0) as ctx:
+        ctx.keep_error_scale(True)
+        for refine in (0.0, 1.0, 1e6):
+            ctx.set_refine(refine)
+            got = ctx.forces(*a, 0, "f32split")
+            G[refine] = ctx.error_scale(n)
+        rows = ctx.last_refine_rows()
+        ref = ctx.forces(*a, 0, "fp64")
+    assert np.isfinite(G[0.0][0]) and all(np.array_equal(G[0.0], g) for g in G.values())
+    assert rows >= 1
+    amag = np.sqrt(ref[0] ** 2 + ref[1] ** 2 + ref[2] ** 2)
+    assert np.sqrt(sum((g[0] - r[0]) ** 2 for g, r in zip(got[:3], ref[:3]))) <= 1e-9 * np.median(amag)
