@@ -68,7 +68,7 @@ namespace sg {
 struct TileBox {          // lo = +inf, hi = -inf: no particle (far from every row)
     float lo[3], hi[3];
     float h2max;
-    float meq;            // FP32 mass of all TJ sources (0: they differ)
+    float meq, meql;      // mass of all TJ sources as float hi + lo (0: they differ)
 };
 
 template <bool NEWTON>
@@ -127,6 +127,16 @@ __device__ __forceinline__ void fold(float *hi, float *lo, f2 v)
     ff_add(h, l, b);
     *hi = h;
     *lo = l;
+}
+// The same for a sum that is still to be multiplied by mh + ml, ml below the
+// last bits of mh; v becomes the product's high part.
+__device__ __forceinline__ void fold_scaled(float *hi, float *lo, f2 &v, float mh, float ml)
+{
+    float a, b;
+    upk(mul2(v, pk(ml, ml)), a, b);
+    v = mul2(v, pk(mh, mh));
+    *lo += a + b;
+    fold(hi, lo, v);
 }
 
 // Near-field pair (r^2 < max H^2) in FP64, folded into the row's
@@ -269,7 +279,7 @@ struct WsSmem {
     static constexpr int META = RAW + NS * RAWSTAGE;       // [NS][NMETA] JMeta (TMA targets)
     static constexpr int COMP = META + NS * NMETA * 32;    // [NS][5][TJ] floats
     static constexpr int BOX = COMP + NS * 5 * TJ * 4;     // [NS] TileBox
-    static constexpr int ACC = BOX + NS * 32;              // [K*8][NT] floats
+    static constexpr int ACC = BOX + (NS * (int)sizeof(TileBox) + 15) / 16 * 16;  // [K*8][NT] floats
     static constexpr int NSB = TJ / (16 * Q);              // 16-source sub-blocks per thread
     static constexpr int NBITS = ACC + K * 8 * NT * 4;     // [K*NSB][NT] ushort near masks
     static constexpr int COOP = NBITS + (K * NSB * NT * 2 + 15) / 16 * 16;  // [W] near_eval buffers
@@ -308,6 +318,15 @@ constexpr int HEAVY_TILES = 4;
 // mass load.  A loop of these pairs alone runs at 2,630 G pairs/s against
 // 2,440 (12 warps, two rows per thread).  The mass-free terms need r within
 // [1e-12, 1e12] to stay in the FP32 range, whatever the masses' unit.
+// All these sums share the FP32 rounding of the mass (up to 2^-24) and the mean
+// relative error of rsqrt.approx (RSQRT_BIAS, measured over all arguments of
+// [1, 4), evenly in log x; largest 1.25e-7), three times that for y^3.  Neither
+// averages out over the tiles, so both go into the low part of the factor,
+// which meets the accumulators' low parts (potentials of a 262K collision, off
+// FP64: 1.4e-8 without it, 8.7e-9 with it, 8.4e-9 with the mass in every term,
+// whose rounding happens to make up for a part; of 200K equal masses 3.2e-8,
+// 8.9e-9, 3.2e-8).  It takes no time (262K 30.3 ms, 1M red giant 490).
+constexpr float RSQRT_BIAS = -5.493e-9f;
 constexpr float EQ_R2_MIN = 1e-24f, EQ_R2_MAX = 1e24f;
 
 // Phase accounting (diagnostic build, -DSG_PHASES): every warp reads clock64
@@ -534,10 +553,12 @@ __global__ void __launch_bounds__((W + NP) * 32) k_f32split(ComputeArgs a)
                     float lo[3] = {INFINITY, INFINITY, INFINITY};
                     float hi[3] = {-INFINITY, -INFINITY, -INFINITY};
                     float h2m = 0.f;
-                    float mlo = INFINITY, mhi = 0.f;  // the records' common masses
+                    double md = 0.0;  // FP64 mass of the record's first source
+                    bool one_mass = true;
                     if (lane < NMETA) {
                         const JMeta M = s_meta[s * NMETA + lane];
-                        mlo = mhi = M.meq;
+                        md = reinterpret_cast<const double *>(stage_raw(s) + 8 * TJ)[lane * META_J];
+                        one_mass = M.meq > 0.f;
                         if (M.ex >= 0.f) {
                             const float c3[3] = {C.chx, C.chy, C.chz};
                             const float mc[3] = {M.cx, M.cy, M.cz}, me[3] = {M.ex, M.ey, M.ez};
@@ -561,13 +582,14 @@ __global__ void __launch_bounds__((W + NP) * 32) k_f32split(ComputeArgs a)
                             hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
                         }
                         h2m = fmaxf(h2m, __shfl_xor_sync(0xffffffffu, h2m, o));
-                        mlo = fminf(mlo, __shfl_xor_sync(0xffffffffu, mlo, o));
-                        mhi = fmaxf(mhi, __shfl_xor_sync(0xffffffffu, mhi, o));
                     }
+                    const double m0 = __shfl_sync(0xffffffffu, md, 0);
+                    one_mass = __all_sync(0xffffffffu, lane >= NMETA || (one_mass && md == m0));
                     if (lane == 0) {
                         TileBox B;
                         B.h2max = h2m;
-                        B.meq = mlo == mhi ? mlo : 0.f;
+                        B.meq = one_mass ? __double2float_rn(m0) : 0.f;
+                        B.meql = one_mass ? __double2float_rn(m0 - (double)B.meq) : 0.f;
                         for (int d = 0; d < 3; d++) { B.lo[d] = lo[d]; B.hi[d] = hi[d]; }
                         s_box[s] = B;
                     }
@@ -714,13 +736,16 @@ __global__ void __launch_bounds__((W + NP) * 32) k_f32split(ComputeArgs a)
                     };
                     if (far && eq) {
                         far_loop(std::true_type{});
-                        const f2 mm = pk(B.meq, B.meq);
+                        const float mh = s_box[s].meq, ml = s_box[s].meql;
+                        constexpr float BIAS = NEWTON ? 0.f : RSQRT_BIAS;
+                        const float m3 = fmaf(mh, -3.f * BIAS, ml), m1 = fmaf(mh, -BIAS, ml);
 #pragma unroll
                         for (int k = 0; k < K; k++) {
-                            tx[k] = mul2(tx[k], mm);
-                            ty[k] = mul2(ty[k], mm);
-                            tz[k] = mul2(tz[k], mm);
-                            tp[k] = mul2(tp[k], mm);
+                            float *acc = s_acc + (k * 8) * NT + tid;
+                            fold_scaled(acc, acc + 4 * NT, tx[k], mh, m3);
+                            fold_scaled(acc + NT, acc + 5 * NT, ty[k], mh, m3);
+                            fold_scaled(acc + 2 * NT, acc + 6 * NT, tz[k], mh, m3);
+                            fold_scaled(acc + 3 * NT, acc + 7 * NT, tp[k], mh, m1);
                         }
                     } else if (far) {
                         far_loop(std::false_type{});
@@ -779,6 +804,7 @@ __global__ void __launch_bounds__((W + NP) * 32) k_f32split(ComputeArgs a)
                         g2[k] = fma2(tx[k], tx[k], g2[k]);
                         g2[k] = fma2(ty[k], ty[k], g2[k]);
                         g2[k] = fma2(tz[k], tz[k], g2[k]);
+                        if (far && eq) continue;  // folded above
                         float *acc = s_acc + (k * 8) * NT + tid;
                         fold(acc, acc + 4 * NT, tx[k]);
                         fold(acc + NT, acc + 5 * NT, ty[k]);

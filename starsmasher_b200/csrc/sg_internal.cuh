@@ -58,7 +58,7 @@ struct JMeta {
     float cx, cy, cz;   // box centre
     float ex, ey, ez;   // half extents (negative: no particle)
     float h2max;
-    float meq;          // FP32 mass that all META_J slots share (0: none, or a pad among them)
+    float meq;          // FP32 rounding of the one mass of all META_J slots (0: masses differ, or a pad)
 };
 // Centre of an i-tile's bounding box as float hi + lo pairs.
 struct ITileMeta {

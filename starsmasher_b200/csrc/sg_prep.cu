@@ -488,11 +488,10 @@ __device__ void record_meta(int r, const SetDesc *sets, const int *meta_set, con
     const int k0 = (r - S.meta_off) * META_J;
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     double h2max = 0.0;
-    float mlo = INFINITY, mhi = 0.f;  // FP32 masses, 0 for a pad
+    const double m0 = k0 < S.n ? D.m[S.poff + k0] : 0.0;
+    bool one_mass = true;
     for (int k = k0 + lane; k < k0 + META_J; k += 32) {
-        const float mk = k < S.n ? __double2float_rn(D.m[S.poff + k]) : 0.f;
-        mlo = fminf(mlo, mk);
-        mhi = fmaxf(mhi, mk);
+        one_mass &= k < S.n && D.m[S.poff + k] == m0;
         if (k < S.n) {
             const int slot = S.poff + k;
             const double v[3] = {D.x[slot], D.y[slot], D.z[slot]};
@@ -511,11 +510,8 @@ __device__ void record_meta(int r, const SetDesc *sets, const int *meta_set, con
             hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        h2max = fmax(h2max, __shfl_xor_sync(0xffffffffu, h2max, o));
-        mlo = fminf(mlo, __shfl_xor_sync(0xffffffffu, mlo, o));
-        mhi = fmaxf(mhi, __shfl_xor_sync(0xffffffffu, mhi, o));
-    }
+    for (int o = 16; o > 0; o >>= 1) h2max = fmax(h2max, __shfl_xor_sync(0xffffffffu, h2max, o));
+    one_mass = __all_sync(0xffffffffu, one_mass);
     if (lane == 0) {
         JMeta M;
         if (lo[0] <= hi[0]) {
@@ -536,7 +532,7 @@ __device__ void record_meta(int r, const SetDesc *sets, const int *meta_set, con
             M.ex = M.ey = M.ez = -1.f;
             M.h2max = 0.f;
         }
-        M.meq = mlo == mhi ? mlo : 0.f;
+        M.meq = one_mass ? __double2float_rn(m0) : 0.f;
         meta[r] = M;
     }
 }

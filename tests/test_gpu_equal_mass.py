@@ -30,3 +30,15 @@ def test_length_units(gpu_ctx, scale):
     ref = gpu_ctx.forces(*a, 0, "fp64")
     e = err_report(*gpu_ctx.forces(*a, 0, "f32split"), *ref)
     assert e["acc_max"] <= 1e-6 and e["pot_max"] <= 1e-6, e
+
+
+@pytest.mark.parametrize("n", [30000, 140000])
+def test_rounding_of_the_mass(gpu_ctx, n):
+    """Potentials per unit mass of a model whose mass FP32 rounds by nearly 2^-24, against
+    those of unit masses: the far tiles, most of the sums, must not share that rounding."""
+    s = inputs.single_polytrope(n, 1.5, seed=4)
+    one = np.ones(n)
+    m = 1.0 + 0.98 * 2.0 ** -24
+    a = gpu_ctx.forces(s.x, s.y, s.z, one, s.range2, 0, "f32split")[3]
+    b = gpu_ctx.forces(s.x, s.y, s.z, m * one, s.range2, 0, "f32split")[3] / m
+    assert abs(np.mean(b / a) - 1.0) <= 0.4 * 2.0 ** -24
