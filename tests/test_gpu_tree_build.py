@@ -48,3 +48,55 @@ def test_parts_of_a_walk(n):
     for g, r, h in zip(got, again, half):
         assert np.array_equal(g, r) and np.array_equal(g[sl], h[sl])
         assert not h[: n // 3].any()
+
+
+# a batch's sets are cut into parts as they are alone: 8 and none, 8 and 2, 4 and 8
+@pytest.mark.parametrize("model", [inputs.single_polytrope, inputs.red_giant])
+@pytest.mark.parametrize("n1, n2", [(1003, 190007), (22999, 100003), (30011, 517)])
+def test_batch_of_mixed_parts(model, n1, n2):
+    a, b = (model(n, seed=n % 89) for n in (n1, n2))
+    f = ("x", "y", "z", "m", "range2")
+    both = [np.concatenate([getattr(a, k), getattr(b, k)]) for k in f]
+    with Context(0) as ctx:
+        ctx.set_theta(0.5)
+        got = ctx.batch_forces([0, n1, n1 + n2], *both, 0, "tree")
+        heavy = ctx.tree_stats()[1]
+        one = ctx.forces(*(getattr(a, k) for k in f), 0, "tree")
+        two = ctx.forces(*(getattr(b, k) for k in f), 0, "tree")
+    alone = [np.concatenate([u, v]) for u, v in zip(one, two)]
+    # the same bits, but for the rows of groups handed to the direct sum, whose
+    # source chunks follow from the call's count of them
+    other = np.flatnonzero(np.any([g != w for g, w in zip(got, alone)], axis=0))
+    assert len(other) <= 32 * heavy
+    amag = np.sqrt(sum(w ** 2 for w in alone[:3]))
+    for g, w in zip(got[:3], alone[:3]):
+        assert (np.abs(g - w)[other] <= 1e-11 * np.median(amag)).all()
+    assert np.allclose(got[3], alone[3], rtol=1e-12)
+
+
+def test_captured_call_with_groups_of_tiny_h():
+    """Groups whose largest H^2 is a subnormal float, which the walking order cannot tell
+    from the unused entries of a captured call's group list, and coincident particles:
+    as the eager call."""
+    import torch
+    n = 3000
+    s = inputs.single_polytrope(n, 1.5, seed=12)
+    a = [getattr(s, k).copy() for k in ("x", "y", "z", "m", "range2")]
+    a[4][:] = 1e-40
+    for v in a[:3]:
+        v[100:200] = v[100]
+    X = [torch.from_numpy(v).cuda() for v in a]
+    out = [torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(4)]
+    with Context(0) as ctx:
+        ctx.set_theta(0.5)
+        ctx.forces_device(n, *X, *out, nkernel=0, precision="tree")
+        ctx.sync()
+        want = [t.cpu().numpy() for t in out]
+        with ctx.capture() as cap:
+            ctx.forces_device(n, *X, *out, nkernel=0, precision="tree")
+        for t in out:
+            t.zero_()
+        torch.cuda.synchronize()
+        cap.graph.launch(1)
+        ctx.sync()
+        assert all(np.array_equal(w, t.cpu().numpy()) for w, t in zip(want, out))
