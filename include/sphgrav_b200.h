@@ -282,8 +282,8 @@ const char *sphgrav_variant_name(int precision, int variant);
  * its only scratch is a static device array of SPHGRAV_NOALLOC_SCRATCH_BYTES
  * that every GPU loading this library holds until the process exits, which
  * caps n at SPHGRAV_NOALLOC_MAX_N (SPHGRAV_ERR_TOO_LARGE beyond).  The first
- * call on a device looks up that array's device address; make that first
- * call before any stream capture.  All calls share the array: calls that
+ * call on a device, of any size, looks up that array's device address and
+ * loads the kernels; make that first call before any stream capture.  All calls share the array: calls that
  * overlap on the GPU (other streams, other host threads) race.  Particle data
  * are not validated (mass > 0 and range2 != 0 are the caller's contract). */
 #define SPHGRAV_NOALLOC_SCRATCH_BYTES (8u << 20)

@@ -294,10 +294,17 @@ extern "C" int sphgrav_forces_fp64_noalloc(int n, const double *x, const double 
     }
     void *part_p = g_noalloc_ptr[dev].load(std::memory_order_acquire);
     if (!part_p) {
-        // set-up on this device's first call (host code cannot use the
-        // symbol's name as a device address)
+        // set-up on this device's first call: the scratch's device address (host
+        // code cannot use the symbol's name as one), and everything that a call of
+        // another size would otherwise load or ask for inside a capture
         void *p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+        for (const void *f : {(const void *)k_fp64_noalloc<1>, (const void *)k_fp64_noalloc<2>,
+                              (const void *)k_merge_noalloc}) {
+            cudaFuncAttributes at;
+            if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, f);
+        }
+        for (int k = 1; k <= 2; k++) noalloc_resident(dev, k);
         if (e != cudaSuccess || !p) {
             cudaGetLastError();
             return SPHGRAV_ERR_CUDA;

@@ -1,6 +1,9 @@
 """The allocation-free call at the edges of its warps, tiles, chunks and of the
 change to two rows per thread, from hardly any near pair to every pair near."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -39,3 +42,43 @@ def test_against_the_context_call(gpu_ctx, n, width):
     assert e["acc_max"] <= 1e-12 and e["pot_max"] <= 1e-12, e
     if n > 4:
         assert np.isfinite(e["acc_max_ill"])
+
+
+_CAPTURE = """
+import ctypes, sys
+import torch
+from starsmasher_b200 import _lib, inputs
+lib = _lib.load()
+def call(n, X, out):
+    assert lib.sphgrav_forces_fp64_noalloc(
+        n, *(ctypes.c_void_p(t.data_ptr()) for t in X), 0, *(ctypes.c_void_p(t.data_ptr()) for t in out),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == _lib.OK
+def model(n):
+    s = inputs.single_polytrope(n, 1.5, seed=n)
+    return ([torch.from_numpy(getattr(s, f)).cuda() for f in ("x", "y", "z", "m", "range2")],
+            torch.zeros(4, n, dtype=torch.float64, device="cuda"))
+first, then = (int(v) for v in sys.argv[1:])
+X, out = model(first)
+call(first, X, out)
+torch.cuda.synchronize()
+X, out = model(then)
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    call(then, X, out)
+assert not out.any()
+graph.replay()
+torch.cuda.synchronize()
+got = out.clone()
+call(then, X, out)
+torch.cuda.synchronize()
+assert torch.equal(got, out) and bool((out[3] < 0).all())
+"""
+
+
+@pytest.mark.parametrize("first, then", [(100, 16384), (16384, 100), (16383, 40000)])
+def test_capture_after_one_call_of_another_size(first, then):
+    """In a process of its own: the first call of any size readies every size for a capture."""
+    env = dict(os.environ, PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    r = subprocess.run([sys.executable, "-c", _CAPTURE, str(first), str(then)], env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
