@@ -25,7 +25,16 @@ namespace sg {
 constexpr int NA_NT = 128;   // threads per block
 constexpr int NA_TJ = 128;   // sources staged per shared-memory tile
 constexpr int NA_MIN_CHUNK = 256;  // sources of a chunk, at least
+constexpr double NA_BIG = 1e150;   // |coordinate| up to which every r^2 is finite
 constexpr size_t NA_SCRATCH_DOUBLES = SPHGRAV_NOALLOC_SCRATCH_BYTES / sizeof(double);
+
+// High word that maybe_near compares r^2 with, for a particle at (x, y, z): its
+// H^2's, or one above every r^2 (infinities and NaN too) past NA_BIG.
+static __device__ __forceinline__ int na_limit(double x, double y, double z, double r2in)
+{
+    const bool fits = fabs(x) <= NA_BIG && fabs(y) <= NA_BIG && fabs(z) <= NA_BIG;
+    return fits ? __double2hiint(fabs(r2in)) : 0x7fffffff;
+}
 
 // Partial sums [chunk][4][n].  Every element a call reads was written earlier
 // in the same call, so nothing needs clearing between calls.
@@ -77,7 +86,8 @@ static __device__ __noinline__ PairOut pair_f64_raw(const double *x, const doubl
 // (mass 0 at r = 1), are flagged 32 sources to a mask and join a queue per warp,
 // which evaluates them 32 at a time, one pair per lane, with the CPU path's
 // formulas; every owner then adds its own results in queue order
-// (deterministic).  The caller's order has no spatial meaning, so a warp meets
+// (deterministic).  Pairs of a particle beyond NA_BIG join it too: r^2 may
+// overflow, where rsqrt_f64 would give NaN.  The caller's order has no spatial meaning, so a warp meets
 // a near pair every few sources: with the pairs evaluated where they are met,
 // each cost the warp ~300 FP64-pipe instructions for one lane's sake.
 template <int K>
@@ -88,7 +98,7 @@ k_fp64_noalloc(int n, const double *x, const double *y, const double *z, const d
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NW = NA_NT / 32;
     __shared__ double s_x[NA_TJ], s_y[NA_TJ], s_z[NA_TJ], s_m[NA_TJ];
-    __shared__ int s_h[NA_TJ];                    // high words of H^2, for maybe_near
+    __shared__ int s_h[NA_TJ];                    // na_limit of the sources
     __shared__ unsigned s_queue[NW][64];          // (source << 6) | row of the warp
     __shared__ unsigned s_owned[NW][K][32];       // entries of the round per owner
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -107,7 +117,7 @@ k_fp64_noalloc(int n, const double *x, const double *y, const double *z, const d
         xi[k] = act[k] ? x[i] : 1e15;
         yi[k] = act[k] ? y[i] : 1e15;
         zi[k] = act[k] ? z[i] : -1e15;
-        hih[k] = act[k] ? __double2hiint(fabs(r2in[i])) : 0;
+        hih[k] = act[k] ? na_limit(xi[k], yi[k], zi[k], r2in[i]) : 0;
         s_owned[warp][k][lane] = 0u;
 #pragma unroll
         for (int q = 0; q < 4; q++) sum[k][q] = acc[k][q] = 0.0;
@@ -169,7 +179,7 @@ k_fp64_noalloc(int n, const double *x, const double *y, const double *z, const d
         s_y[tid] = has ? ny : -1e15;
         s_z[tid] = has ? nz : 1e15;
         s_m[tid] = has ? nm : 0.0;
-        s_h[tid] = has ? __double2hiint(fabs(nh)) : 0;
+        s_h[tid] = has ? na_limit(nx, ny, nz, nh) : 0;
         __syncthreads();
         fetch(jt + NA_TJ);
         const int blocks = min(NA_TJ / 32, (j1 - jt + 31) / 32);

@@ -44,6 +44,33 @@ def test_against_the_context_call(gpu_ctx, n, width):
         assert np.isfinite(e["acc_max_ill"])
 
 
+@pytest.mark.parametrize("n", [129, 300, 16400])
+def test_separations_whose_square_overflows(n):
+    """Two particles farther away than 1e154: no force and no potential, as 1/r underflows."""
+    import torch
+    s = inputs.single_polytrope(n, 1.5, seed=n)
+    a = [getattr(s, f).copy() for f in ("x", "y", "z", "m", "range2")]
+    a[4][-1] = -a[4][-1]  # no potential of its own
+
+    def call(*a):
+        k = len(a[0])
+        X = [torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in a]
+        out = [torch.zeros(k, dtype=torch.float64, device="cuda") for _ in range(4)]
+        st = _lib.load().sphgrav_forces_fp64_noalloc(
+            k, *(ctypes.c_void_p(t.data_ptr()) for t in X), 0,
+            *(ctypes.c_void_p(t.data_ptr()) for t in out),
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == _lib.OK
+        return [t.cpu().numpy() for t in out]
+
+    ref = call(*(v[1:-1] for v in a))
+    a[0][-1], a[1][0] = 1e160, -1e200
+    got = call(*a)
+    e = err_report(*(v[1:-1] for v in got), *ref)
+    assert e["acc_max"] <= 1e-12 and e["pot_max"] <= 1e-12, e
+    assert all(v[-1] == 0.0 for v in got)
+
+
 _CAPTURE = """
 import ctypes, sys
 import torch
