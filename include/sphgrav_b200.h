@@ -299,7 +299,8 @@ const char *sphgrav_status_string(int status);
 const char *sphgrav_last_error_message(void);
 /* Kernels launched by this library since the process started. */
 unsigned long long sphgrav_launch_count(void);
-/* Work items and j-chunks of the last computation (for tests and tuning). */
+/* Work items and j-chunks of the last computation (for tests and tuning; a tree
+ * call has no items). */
 int sphgrav_last_plan_info(sphgrav_ctx *ctx, int *nitems, int *nchunks_max,
                            int *variant);
 /* The work plan a call on whole sets would use, computed on the host only

@@ -410,6 +410,25 @@ static int choose_variant(sphgrav_ctx *c, int precision, const std::vector<int> 
 }
 
 // ------------------------------------------------------------------ plan
+// Curve-key bits per axis.  The octree's levels are the key's 3-bit digits, so
+// tree calls keep 21.  For the direct sums every 8 key bits cost the sort a
+// pass, which matters only for small sets: up to 65,536 particles they take
+// cells just fine enough that particles rarely share one (2^(3b) cells, about
+// 2^15 per particle, at least 2^10 per axis; 16K: 4 passes instead of 8).
+// Larger sets keep 21 bits: a curve of another order has another orientation,
+// so it tiles a centred star differently (on the 1M red giant 18 refined rows
+// instead of 8, RMS error 6.2e-8 instead of 4.7e-8), for a sort that is < 0.1%
+// of the call.
+static void curve_bits(Plan &P)
+{
+    const int setbits = ceil_log2(std::max(1, P.nsets));
+    const int want = (P.tree || P.max_n > 65536)
+                         ? 21
+                         : std::max(10, (ceil_log2(std::max(2, P.max_n)) + 2) / 3 + 5);
+    P.bits = std::min(std::min(21, want), (64 - setbits) / 3);
+    P.end_bit = 3 * P.bits + setbits;
+}
+
 // The work plan of one call: host-only arithmetic (resident = persistent CTAs
 // of the variant on the device), so it also runs without a GPU
 // (sphgrav_plan_preview).
@@ -440,12 +459,12 @@ static int build_plan(int resident, const std::vector<int> &offsets, bool full_r
         d.ni = full_rows ? d.n : ni;
         d.i_lo = full_rows ? 0 : i_lo;
         d.tile_off = (int)toff;
-        d.ntiles = (d.ni + P.itile - 1) / P.itile;
+        d.ntiles = tree ? 0 : (d.ni + P.itile - 1) / P.itile;
         d.meta_off = (int)moff;
         poff += d.npad;
         ioff += d.ni;
         toff += d.ntiles;
-        moff += d.npad / META_J;
+        moff += tree ? 0 : d.npad / META_J;
         P.max_n = std::max(P.max_n, d.n);
         P.max_npad = std::max(P.max_npad, d.npad);
         P.sets.push_back(d);
@@ -456,6 +475,11 @@ static int build_plan(int resident, const std::vector<int> &offsets, bool full_r
     P.rows_tot = (int)ioff;
     P.ntiles = (int)toff;
     P.nmeta = (int)moff;
+    curve_bits(P);
+    if (tree) {  // the walk has no row tiles: the sets alone
+        P.valid = true;
+        return SPHGRAV_OK;
+    }
     const int target = 4 * resident;
     const int min_chunk = min_chunk_sources(precision, P.max_n);
     // One set: items are all alike, so pick the chunk count whose item count
@@ -605,21 +629,6 @@ static int build_plan(int resident, const std::vector<int> &offsets, bool full_r
     P.nitems = (int)P.items.size();
     P.nslots = slot;
     P.grid = std::max(1, std::min(P.nitems, resident));
-    const int setbits = ceil_log2(std::max(1, P.nsets));
-    // Curve-key bits per axis.  The octree's levels are the key's 3-bit
-    // digits, so tree calls keep 21.  For the direct sums every 8 key bits
-    // cost the sort a pass, which matters only for small sets: up to 65,536
-    // particles they take cells just fine enough that particles rarely
-    // share one (2^(3b) cells, about 2^15 per particle, at least 2^10 per
-    // axis; 16K: 4 passes instead of 8).  Larger sets keep 21 bits: a curve
-    // of another order has another orientation, so it tiles a centred star
-    // differently (on the 1M red giant 18 refined rows instead of 8, RMS
-    // error 6.2e-8 instead of 4.7e-8), for a sort that is < 0.1% of the call.
-    const int want = (tree || P.max_n > 65536)
-                         ? 21
-                         : std::max(10, (ceil_log2(std::max(2, P.max_n)) + 2) / 3 + 5);
-    P.bits = std::min(std::min(21, want), (64 - setbits) / 3);
-    P.end_bit = 3 * P.bits + setbits;
     P.valid = true;
     return SPHGRAV_OK;
 }
@@ -680,7 +689,7 @@ static int prepare(sphgrav_ctx *c, const std::vector<int> &offsets, bool full_ro
     TRY(ensure(c, c->keys_out, nt, "keys"));
     TRY(ensure(c, c->vals_in, nt, "vals"));
     TRY(ensure(c, c->vals_out, nt, "vals"));
-    TRY(ensure(c, c->ilist, std::max(1, P.rows_tot), "rows"));
+    if (!P.tree) TRY(ensure(c, c->ilist, std::max(1, P.rows_tot), "rows"));
     if (6 * (size_t)std::max(1, P.nsets) > c->bbox.cap) {
         TRY(ensure(c, c->bbox, 6 * (size_t)std::max(1, P.nsets), "bbox"));
         // the state that every call leaves behind (launch_gather)
@@ -713,7 +722,7 @@ static int prepare(sphgrav_ctx *c, const std::vector<int> &offsets, bool full_ro
     }
     if (!sorts_in_tiles(P.ntot))
         TRY(ensure(c, c->sort_temp, std::max<size_t>(sort_temp_bytes(P.ntot, P.end_bit), 1), "sort temp"));
-    if (!P.full_rows) {
+    if (!P.full_rows && !P.tree) {
         const size_t selb = select_temp_bytes(P.ntot);
         TRY(ensure(c, c->sel_temp, std::max<size_t>(selb, 1), "select temp"));
     }

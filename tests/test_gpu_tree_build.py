@@ -100,3 +100,21 @@ def test_captured_call_with_groups_of_tiny_h():
         cap.graph.launch(1)
         ctx.sync()
         assert all(np.array_equal(w, t.cpu().numpy()) for w, t in zip(want, out))
+
+
+def test_no_direct_sum_plan():
+    """The walk has no row tiles: a tree call plans no work items, and one of other rows of
+    the same set gives the same bits."""
+    s = inputs.single_polytrope(20011, 1.5, seed=2)
+    a = (s.x, s.y, s.z, s.m, s.range2)
+    with Context(0) as ctx:
+        full = ctx.forces(*a, 0, "tree")
+        assert ctx.plan_info()["nitems"] == 0
+        part = ctx.forces(*a, 0, "tree", 4000, 5000)
+        direct = ctx.forces(*a, 0, "f32split")
+        assert ctx.plan_info()["nitems"] > 0
+        again = ctx.forces(*a, 0, "tree")
+        with Context(0) as other:
+            assert all(np.array_equal(u, v) for u, v in zip(direct, other.forces(*a, 0, "f32split")))
+    for u, v, w in zip(full, part, again):
+        assert np.array_equal(u, w) and np.array_equal(u[4000:9000], v[4000:9000])
