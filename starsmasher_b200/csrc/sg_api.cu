@@ -139,6 +139,7 @@ struct Plan {
     bool tree = false;  // Barnes-Hut call: the octree's levels are the full curve key
     // derived
     int nsets = 0, ntot = 0, npad_tot = 0, rows_tot = 0, ntiles = 0, nmeta = 0, nitems = 0;
+    long long res_slots = 0;  // tree: tree_res_slots of all sets
     int nslots = 0, itile = 0, tj = 0, max_n = 0, max_npad = 0, bits = 21, end_bit = 63;
     int grid = 1, nchunks_max = 1;
     std::vector<SetDesc> sets;
@@ -462,6 +463,8 @@ static int build_plan(int resident, const std::vector<int> &offsets, bool full_r
         d.tile_off = (int)toff;
         d.ntiles = tree ? 0 : (d.ni + P.itile - 1) / P.itile;
         d.meta_off = (int)moff;
+        d.res_off = P.res_slots;
+        if (tree) P.res_slots += tree_res_slots(d.n, d.npad);
         poff += d.npad;
         ioff += d.ni;
         toff += d.ntiles;
@@ -935,7 +938,7 @@ static int run_tree(sphgrav_ctx *c, const std::vector<int> &offsets, bool full_r
     int nparts = 1;
     for (const SetDesc &d : P.sets)
         if (d.n > 0) nparts = std::max(nparts, tree_walk_parts(d.n));
-    TRY(ensure(c, c->tres, 4 * (size_t)nslots * nparts, "tree results"));
+    TRY(ensure(c, c->tres, 4 * (size_t)P.res_slots, "tree results"));
     TRY(ensure(c, c->tgtaken, (size_t)n, "tree groups"));
     // heavy groups' partial sums: room for TREE_HEAVY_CAP groups (a captured
     // call's bound), more when an eager call finds more
@@ -945,7 +948,7 @@ static int run_tree(sphgrav_ctx *c, const std::vector<int> &offsets, bool full_r
     a.geom = c->tgeom.p;
     a.mp = c->tmp.p;
     a.D = D;
-    a.n = nslots;
+    a.sets = c->sets.p;
     a.ngroups = ng.host;
     a.ngroups_dev = ng.dev;
     a.nroots = nsets;
@@ -987,15 +990,15 @@ static int run_tree(sphgrav_ctx *c, const std::vector<int> &offsets, bool full_r
     if (dev || nheavy > 0) {
         const int hcap = dev ? TREE_HEAVY_CAP : std::max(nheavy, TREE_HEAVY_CAP);
         CUDA_TRY(tree_heavy(dev ? 0 : nheavy, c->tgcount.p + 1, hcap, c->theavy.p, c->tgorder.p,
-                            c->tnodes.p, nsets, D, nslots, P.max_n, nkernel, nparts,
-                            c->theavy_part.p, c->tres.p, c->err.p, st));
+                            c->sets.p, c->tnodes.p, nsets, D, P.max_n, nkernel, c->theavy_part.p,
+                            c->tres.p, c->err.p, st));
     }
     c->tree_groups_last = dev ? -1 : ng.host;
     c->tree_heavy_last = nheavy;
     if (timed) CUDA_TRY(cudaEventRecord(c->prof_events[c->prof_used++].second, st));
     if (W) TRY(ensure(c, c->twsum, (size_t)nsets * tree_scatter_blocks(P.max_n), "tree W sums"));
-    CUDA_TRY(tree_scatter(c->sets.p, nsets, P.max_n, nslots, nparts, full_rows ? 0 : i_lo,
-                          full_rows ? n : ni, c->tres.p, D, out, c->twsum.p, W, st));
+    CUDA_TRY(tree_scatter(c->sets.p, nsets, P.max_n, full_rows ? 0 : i_lo, full_rows ? n : ni,
+                          c->tres.p, D, out, c->twsum.p, W, st));
     return SPHGRAV_OK;
 }
 

@@ -29,6 +29,7 @@ struct SetDesc {
     int nchunks;   // j-chunks per i-tile (the main plan: the most of any tile)
     int light_off; // refine plans, sets with few listed rows: first row-chunk item
     int light_nch; // ... and source chunks per row (0: the set's rows use tiles)
+    long long res_off;  // tree plans: first slot of the set's results, [part][4][npad] doubles
 };
 
 // One unit of the persistent kernels' device-side queue.

@@ -298,9 +298,10 @@ struct TreeWalkArgs {
     const NodeGeom *geom;
     const NodeMP *mp;
     SortedF64 D;
-    int n, ngroups, nkernel;   // n: result stride (sorted slots, pads included)
+    int ngroups, nkernel;
     const int *ngroups_dev;    // when non-null the group count is read here
     int nroots;                // roots are nodes [0, nroots), one per set
+    const SetDesc *sets;
     const int2 *groups;  // [ngroups] sorted-slot ranges (start, end), end - start <= 32
     int *head;       // group counter (zeroed before the launch)
     int *heavy;      // [ngroups] groups handed to the direct sum ...
@@ -311,7 +312,7 @@ struct TreeWalkArgs {
     const int *parent;  // per node
     const int *lv;   // level table of the build
     int *gtaken;     // [ngroups] tested-list entries per group (zeroed before the launch)
-    double *out;     // [nparts][4][n] in sorted order
+    double *out;     // the sets' results (SetDesc::res_off), in sorted order
     int *err;
 };
 size_t tree_scan_temp_bytes(int n);
@@ -343,19 +344,27 @@ cudaError_t tree_props(DevCount nn, const TreeNode *nodes, const int *parent, in
                        cudaStream_t st);
 int tree_walk_warps(int sm_count);
 cudaError_t tree_walk(const TreeWalkArgs &a, int sm_count, cudaStream_t st);
+// Slots of the sets' results: a set has as many parts as its own walk, however
+// many the largest count in the batch is.
+inline long long tree_res_slots(int n, int npad) { return (long long)npad * tree_walk_parts(n); }
+// Where quantity q of part p of the set's sorted slot `slot` is in the results.
+__host__ __device__ inline size_t tree_res_at(const SetDesc &S, int p, int q, int slot)
+{
+    return 4 * (size_t)S.res_off + ((size_t)p * 4 + q) * S.npad + (slot - S.poff);
+}
 // Rows [i_lo, i_lo + ni) to the caller's order, the parts added in order; W of
 // every set (nullable) through wpart, nsets * tree_scatter_blocks(max_n) doubles.
 int tree_scatter_blocks(int max_n);
-cudaError_t tree_scatter(const SetDesc *sets, int nsets, int max_n, int nslots, int nparts, int i_lo,
-                         int ni, const double *res, const SortedF64 &D, const OutputsDev &out,
+cudaError_t tree_scatter(const SetDesc *sets, int nsets, int max_n, int i_lo, int ni,
+                         const double *res, const SortedF64 &D, const OutputsDev &out,
                          double *wpart, double *W, cudaStream_t st);
 // Direct FP64 sums over the group's own set for the groups the walk handed
 // over (*nheavy on the device, at most `cap`; more set DEVERR_TREE_CAP).
 // max_n: the largest set; nheavy_host > 0 sizes the grid exactly.
 cudaError_t tree_heavy(int nheavy_host, const int *nheavy, int cap, const int *heavy,
-                       const int2 *groups, const TreeNode *nodes, int nroots, const SortedF64 &D,
-                       int nslots, int max_n, int nkernel, int nparts, double *partials,
-                       double *out, int *err, cudaStream_t st);
+                       const int2 *groups, const SetDesc *sets, const TreeNode *nodes, int nroots,
+                       const SortedF64 &D, int max_n, int nkernel, double *partials, double *out,
+                       int *err, cudaStream_t st);
 // Partial-sum doubles tree_heavy needs for up to `cap` heavy groups.
 size_t tree_heavy_partials(int cap, int max_n);
 // Raises DEVERR_TREE_CAP when the build ran out of nodes (lv overflow flag).

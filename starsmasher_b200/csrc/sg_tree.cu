@@ -809,11 +809,12 @@ __global__ void __launch_bounds__(WALK_WARPS * 32, 5) k_tree_walk(const __grid_c
         if (heavy || report()) continue;
         if (overflow && lane == 0) atomicOr(a.err, DEVERR_TREE);
         if (act) {
-            double *o = a.out + (size_t)part * 4 * a.n + s;
+            const SetDesc S = a.sets[root];
+            double *o = a.out + tree_res_at(S, part, 0, s);
             o[0] = fx;
-            o[(size_t)a.n] = fy;
-            o[2 * (size_t)a.n] = fz;
-            o[3 * (size_t)a.n] = fp;
+            o[(size_t)S.npad] = fy;
+            o[2 * (size_t)S.npad] = fz;
+            o[3 * (size_t)S.npad] = fp;
         }
     }
 }
@@ -878,8 +879,8 @@ k_tree_heavy(const int *nheavy_p, int cap, const int *heavy, const int2 *groups,
 constexpr int HEAVY_MERGE_SLICES = 8;
 __global__ void __launch_bounds__(4 * HEAVY_MERGE_SLICES * 32)
 k_tree_heavy_merge(const int *nheavy_p, int cap, const int *heavy,
-                   const int2 *groups, int max_n, const double *partials, int nslots, int nparts,
-                   double *out)
+                   const int2 *groups, const SetDesc *sets, const TreeNode *nodes, int nroots,
+                   int max_n, const double *partials, double *out)
 {
     __shared__ double s_sum[HEAVY_MERGE_SLICES][4][32];
     const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) & 3, slice = threadIdx.x >> 7;
@@ -897,8 +898,9 @@ k_tree_heavy_merge(const int *nheavy_p, int cap, const int *heavy,
         __syncthreads();
         if (slice != 0 || si >= grp.y) continue;
         for (int k = 1; k < HEAVY_MERGE_SLICES; k++) v += s_sum[k][q][lane];
-        out[(size_t)q * nslots + si] = v;
-        for (int p = 1; p < nparts; p++) out[((size_t)p * 4 + q) * nslots + si] = 0.0;
+        const SetDesc S = sets[nroots > 1 ? root_of(nodes, nroots, grp.x) : 0];
+        out[tree_res_at(S, 0, q, si)] = v;
+        for (int p = 1; p < tree_walk_parts(S.n); p++) out[tree_res_at(S, p, q, si)] = 0.0;
     }
 }
 
@@ -910,9 +912,9 @@ size_t tree_heavy_partials(int cap, int max_n)
 }
 
 cudaError_t tree_heavy(int nheavy_host, const int *nheavy, int cap, const int *heavy,
-                       const int2 *groups, const TreeNode *nodes, int nroots, const SortedF64 &D,
-                       int nslots, int max_n, int nkernel, int nparts, double *partials,
-                       double *out, int *err, cudaStream_t st)
+                       const int2 *groups, const SetDesc *sets, const TreeNode *nodes, int nroots,
+                       const SortedF64 &D, int max_n, int nkernel, double *partials, double *out,
+                       int *err, cudaStream_t st)
 {
     // eager calls know the count: one block per (group, chunk); captured
     // calls size the grid for the most chunks any count can give
@@ -923,8 +925,8 @@ cudaError_t tree_heavy(int nheavy_host, const int *nheavy, int cap, const int *h
                                                      max_n, nkernel, partials, err);
     ++g_launches;
     const int mblocks = nheavy_host > 0 ? std::min(nheavy_host, cap) : 256;
-    k_tree_heavy_merge<<<mblocks, 4 * HEAVY_MERGE_SLICES * 32, 0, st>>>(nheavy, cap, heavy, groups, max_n,
-                                                                       partials, nslots, nparts, out);
+    k_tree_heavy_merge<<<mblocks, 4 * HEAVY_MERGE_SLICES * 32, 0, st>>>(
+        nheavy, cap, heavy, groups, sets, nodes, nroots, max_n, partials, out);
     ++g_launches;
     return cudaGetLastError();
 }
@@ -934,13 +936,13 @@ cudaError_t tree_heavy(int nheavy_host, const int *nheavy, int cap, const int *h
 // the set's slots (a contiguous run, in a fixed order) for W.
 constexpr int SCATTER_NT = 256;
 __global__ void __launch_bounds__(SCATTER_NT)
-k_tree_scatter(const SetDesc *sets, int nsets, int nslots, bool split, int i_lo, int ni,
-               const double *res, SortedF64 D, OutputsDev out, double *wpart)
+k_tree_scatter(const SetDesc *sets, int nsets, int i_lo, int ni, const double *res,
+               SortedF64 D, OutputsDev out, double *wpart)
 {
     __shared__ double s_w[SCATTER_NT];
     for (int set = blockIdx.y; set < nsets; set += gridDim.y) {
         const SetDesc S = sets[set];
-        const int nparts = split ? tree_walk_parts(S.n) : 1;
+        const int nparts = tree_walk_parts(S.n);
         const int per = ((S.n + gridDim.x - 1) / gridDim.x + SCATTER_NT - 1) / SCATTER_NT * SCATTER_NT;
         const int k0 = min(S.n, (int)min((long long)S.n, (long long)blockIdx.x * per));
         const int k1 = min(S.n, k0 + per);
@@ -949,10 +951,10 @@ k_tree_scatter(const SetDesc *sets, int nsets, int nslots, bool split, int i_lo,
             const int s = S.poff + k;
             double v[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) v[q] = res[(size_t)q * nslots + s];
+            for (int q = 0; q < 4; q++) v[q] = res[tree_res_at(S, 0, q, s)];
             for (int p = 1; p < nparts; p++) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) v[q] += res[((size_t)p * 4 + q) * nslots + s];
+                for (int q = 0; q < 4; q++) v[q] += res[tree_res_at(S, p, q, s)];
             }
             w += D.m[s] * v[3];
             const int o = D.orig[s];
@@ -1117,13 +1119,13 @@ int tree_scatter_blocks(int max_n)
     return std::max(1, std::min((max_n + SCATTER_NT - 1) / SCATTER_NT, 1024));
 }
 
-cudaError_t tree_scatter(const SetDesc *sets, int nsets, int max_n, int nslots, int nparts, int i_lo,
-                         int ni, const double *res, const SortedF64 &D, const OutputsDev &out,
+cudaError_t tree_scatter(const SetDesc *sets, int nsets, int max_n, int i_lo, int ni,
+                         const double *res, const SortedF64 &D, const OutputsDev &out,
                          double *wpart, double *W, cudaStream_t st)
 {
     const int nb = tree_scatter_blocks(max_n);
     k_tree_scatter<<<dim3(nb, grid_sets(nsets)), SCATTER_NT, 0, st>>>(
-        sets, nsets, nslots, nparts > 1, i_lo, ni, res, D, out, W ? wpart : nullptr);
+        sets, nsets, i_lo, ni, res, D, out, W ? wpart : nullptr);
     ++g_launches;
     if (W) {
         k_tree_wsum<<<nsets, SCATTER_NT, 0, st>>>(nb, wpart, W);

@@ -118,3 +118,25 @@ def test_no_direct_sum_plan():
             assert all(np.array_equal(u, v) for u, v in zip(direct, other.forces(*a, 0, "f32split")))
     for u, v, w in zip(full, part, again):
         assert np.array_equal(u, w) and np.array_equal(u[4000:9000], v[4000:9000])
+
+
+def test_memory_of_a_small_set_beside_a_large_one():
+    """The parts of a small set's walk cost its own results' memory, not the batch's."""
+    import torch
+    n, small = 400000, 300
+    s = inputs.single_polytrope(n + small, 1.5, seed=1)
+    X = [torch.from_numpy(getattr(s, k)).cuda() for k in ("x", "y", "z", "m", "range2")]
+    out = [torch.zeros(n + small, dtype=torch.float64, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+
+    def used(offsets):
+        free = torch.cuda.mem_get_info()[0]
+        with Context(0) as ctx:
+            ctx.set_theta(0.7)
+            ctx.batch_forces_device(offsets, *X, *out, nkernel=0, precision="tree")
+            ctx.sync()
+            return free - torch.cuda.mem_get_info()[0]
+
+    used([0, n])  # loads the kernels
+    one = used([0, n])
+    assert used([0, n, n + small]) - one < 0.2 * one
