@@ -323,7 +323,7 @@ int sphgrav_profile_read(sphgrav_ctx *ctx, double *kernel_ms, int *launches);
  * SPHGRAV_ERR_UNSUPPORTED).  While sphgrav_profile_enable is on, every
  * split-FP32 launch adds the SM cycles its warps spend per phase; this call
  * synchronises the stream, copies the 16 counters and zeroes them.  Order:
- * consumer item fetch + barrier, row loads, waits for a staged tile, far loop,
+ * consumer waits for an item, row loads, waits for a staged tile, far loop,
  * checked loop, FP64 near pairs, item end; producer waits, producer work;
  * then counts of far and checked (warp, tile) pairs, near_eval calls and
  * items per consumer warp.  No counterpart in the reference. */

@@ -115,7 +115,7 @@ struct ComputeArgs {
 // kernel compiled with -DSG_PHASES).  Consumer and producer warps sum the
 // SM cycles they spend in each phase; counts are per warp.
 enum Phase {
-    PH_ITEM = 0,      // consumer: queue fetch and the CTA barrier at an item start
+    PH_ITEM = 0,      // consumer: waiting for the next item
     PH_ROWS,          // consumer: loading the item's rows, warp box
     PH_WAIT_FULL,     // consumer: waiting for a staged tile
     PH_FAR,           // consumer: far loop + tile fold

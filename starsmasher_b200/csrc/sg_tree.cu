@@ -1049,7 +1049,7 @@ cudaError_t tree_groups(DevCount nn, int nroots, const TreeNode *nodes, const in
 // is tested pair by pair, so those groups walk longest; started first, they
 // do not leave one warp running after the rest (results do not depend on the
 // order: each group's sums are its own).  Entries past the group count (a
-// device count bounded by ng.host) get key 0 and sort last.
+// device count bounded by ng.host) have key 0 and sort last.
 __global__ void k_tree_group_keys(DevCount ngc, int bound, const int2 *glist, const double *h2,
                                   unsigned *keys)
 {
@@ -1061,9 +1061,10 @@ __global__ void k_tree_group_keys(DevCount ngc, int bound, const int2 *glist, co
         const int2 r = glist[g];
         for (int s = r.x; s < r.y; s++) m = fmax(m, h2[s]);
     }
-    // non-negative floats order as their bits; a group always keys above
-    // the unused entries, even if its H^2 rounds to a float 0
-    keys[g] = g < ng ? max(__float_as_uint((float)m), 1u) : 0u;
+    // non-negative floats order as their bits, the exponents alone sorted; a
+    // group whose H^2 has none (a subnormal float) ties with the unused entries,
+    // which the stable sort leaves behind it
+    keys[g] = g < ng ? __float_as_uint((float)m) : 0u;
 }
 
 size_t tree_order_temp_bytes(int ng)
