@@ -933,7 +933,7 @@ static int run_tree(sphgrav_ctx *c, const std::vector<int> &offsets, bool full_r
     CUDA_TRY(tree_order_groups(ng, c->tglist.p, c->tgorder.p, D.h2, (unsigned *)c->tcnt.p,
                                (unsigned *)c->toff.p, c->tscan.p, c->tscan.cap, st));
     CUDA_TRY(tree_props(nn, c->tnodes.p, c->tparent.p, c->tdone.p, D, c->theta, c->tacc.p,
-                        c->tgeom.p, c->tmp.p, st));
+                        c->tgeom.p, c->tmp.p, c->sm_count, st));
     TRY(ensure(c, c->tstack, (size_t)tree_walk_warps(c->sm_count) * TREE_STACK, "tree stack"));
     int nparts = 1;
     for (const SetDesc &d : P.sets)

@@ -341,7 +341,7 @@ cudaError_t tree_order_groups(DevCount ng, const int2 *glist, int2 *ordered, con
 size_t tree_acc_bytes(int nn);
 cudaError_t tree_props(DevCount nn, const TreeNode *nodes, const int *parent, int *done,
                        const SortedF64 &D, double theta, void *acc_buf, NodeGeom *geom, NodeMP *mp,
-                       cudaStream_t st);
+                       int sm_count, cudaStream_t st);
 int tree_walk_warps(int sm_count);
 cudaError_t tree_walk(const TreeWalkArgs &a, int sm_count, cudaStream_t st);
 // Slots of the sets' results: a set has as many parts as its own walk, however

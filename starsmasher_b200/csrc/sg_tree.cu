@@ -1095,9 +1095,9 @@ size_t tree_acc_bytes(int nn) { return (size_t)nn * sizeof(NodeAcc); }
 
 cudaError_t tree_props(DevCount nn, const TreeNode *nodes, const int *parent, int *done,
                        const SortedF64 &D, double theta, void *acc_buf, NodeGeom *geom, NodeMP *mp,
-                       cudaStream_t st)
+                       int sm_count, cudaStream_t st)
 {
-    k_tree_props<<<grid_for(nn, 8, 148 * 16), 256, 0, st>>>(nn, nodes, parent, done, D, theta,
+    k_tree_props<<<grid_for(nn, 8, sm_count * 16), 256, 0, st>>>(nn, nodes, parent, done, D, theta,
                                                             (NodeAcc *)acc_buf, geom, mp);
     ++g_launches;
     return cudaGetLastError();
