@@ -380,9 +380,9 @@ static int choose_variant(sphgrav_ctx *c, int precision, const std::vector<int> 
     //                                 1.70, red giant 1.65 vs 1.77; 90K 4.32 vs
     //                                 5.02).  Batches keep W12K1Q4 there: over ten
     //                                 batches with a mean of 2^14 the 192-row tiles
-    //                                 round 3% more on average (2-norms against
-    //                                 FP64; 40 of 12K-24K 3.73e-8 vs 3.56e-8),
-    //                                 for 8.2 ms a call instead of 9.1
+    //                                 round 10% more on average (2-norms against
+    //                                 FP64; 40 of 12K-24K 2.95e-8 vs 2.64e-8),
+    //                                 for 8.4 ms a call instead of 9.2
     //   from 2^13: W12K1Q4, 7 stages (8K: 0.135 vs 0.142; 16K: 0.307 vs 0.302
     //                                 for W15K1Q2, whose 240-row tiles leave 69
     //                                 rows for the FP64 refine against 22: whole
@@ -390,7 +390,7 @@ static int choose_variant(sphgrav_ctx *c, int precision, const std::vector<int> 
     //   below    W8K1Q4              (whole calls; 2,000: 88 us vs 94 for
     //                                 W12K1Q4; 5,003: 181 vs 161, but red giant
     //                                 187 vs 226: more rows refined.  Batches: 64
-    //                                 of 1K-4K 0.93 ms vs 0.79 for W12K1Q4, whose
+    //                                 of 1K-4K 0.94 ms vs 0.80 for W12K1Q4, whose
     //                                 96-row tiles round 2% more on average)
     // Twelve consumer warps put the same number of consumers on every SMSP;
     // all without the Newton step on rsqrt.approx: in FP32 the step's own
